@@ -1,0 +1,45 @@
+// Programmatic dependent launch: a kernel launched with `pdl_launch(..., dependent = true)` may start while its
+// predecessor in the stream still runs, once every CTA of the predecessor has executed pdl_trigger() (or exited).
+// It must execute pdl_wait() before it touches anything the predecessor writes or reads; the wait returns when the
+// predecessor has completed and its memory is visible, and because every kernel of such a chain waits before it
+// finishes, so has everything launched before it.  Both instructions do nothing in a kernel launched the ordinary way.
+//
+// A kernel that allocates TMEM triggers after its allocation: its dependents are then only resident beside CTAs that
+// already own their columns, so an allocation can never wait for a CTA that waits for it.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace dz {
+
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launch with an optional cluster of `cluster_x` CTAs along x, optionally as a programmatic dependent.
+template <class... Params, class... Args>
+inline cudaError_t pdl_launch(void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                              int cluster_x, bool dependent, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (cluster_x > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster_x;
+    attr[n].val.clusterDim.y = 1;
+    attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (dependent) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kern, Params(args)...);
+}
+
+}  // namespace dz

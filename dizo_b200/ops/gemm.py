@@ -20,6 +20,7 @@ ACT = {None: 0, "none": 0, "relu": 1, "gelu": 2}
 _VARIANT = int(os.environ.get("DIZO_GEMM_VARIANT", "0"))
 # 0: SwiGLU as a GEMM followed by the stand-alone silu_mul kernel (for A/B measurements)
 _SWIGLU_FUSED = os.environ.get("DIZO_SWIGLU_FUSED", "1") != "0"
+SKINNY_ROWS = 64       # the row limit of csrc/skinny_sm100.cu
 _ROPE_FUSED = os.environ.get("DIZO_ROPE_FUSED", "1") != "0"
 
 
@@ -52,6 +53,12 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor) -> torch.Tensor:
     F = N // 2
     x2 = x.reshape(-1, K)
     M = x2.shape[0]
+    if _SWIGLU_FUSED and x.is_cuda and _VARIANT == 0 and 0 < M <= SKINNY_ROWS:
+        assert x.dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 and w_gate_up.stride(-1) == 1
+        x2 = x2 if x2.stride(-1) == 1 else x2.contiguous()
+        out = torch.empty((M, F), dtype=torch.bfloat16, device=x.device)
+        _skinny(x2, w_gate_up, out, None, None, 3, 1.0)
+        return out.reshape(*x.shape[:-1], F)
     fused = (_SWIGLU_FUSED and x.is_cuda and _VARIANT in (0, 2) and N % 256 == 0 and M >= 256
              and ((M + 255) // 256) * (N // 256) >= 48)
     if not fused:
@@ -98,6 +105,27 @@ def linear_qkv_rope(x: torch.Tensor, w_qkv: torch.Tensor, L: int, pos0: int, H: 
     return out
 
 
+def _skinny_pays(M: int, N: int) -> bool:
+    """Whether the swapped-operand, K-split kernel takes a product with M rows and N columns.  Up to 16 rows it always
+    wins (one row, us, 128-row tiles / skinny: N 2048 K 8192 32.9 / 10.5, N 50272 K 2048 59.1 / 36.3).  With more rows its
+    wider activation operand costs L2 traffic per tile of W, which only K splitting makes up for: at 32 rows N 32000 K
+    4096 50.2 / 48.1 but N 50272 K 2048 40.6 / 42.8; at 64 rows N 2048 K 8192 31.9 / 13.7, N 8192 K 2048 12.4 / 11.9, but
+    N 16384 K 4096 29.2 / 29.6 and N 50272 K 2048 40.4 / 49.5."""
+    tiles = (N + 127) // 128
+    return 0 < M <= 16 or (M <= 32 and tiles <= 296) or (M <= SKINNY_ROWS and tiles <= 74)
+
+
+def _skinny(x2, w, out2, bias, res2, act: int, scale: float, splits: int = 0) -> None:
+    """``out2 = epilogue(x2 @ w.T)`` for at most ``SKINNY_ROWS`` rows (``act`` 3: SwiGLU over gate | up rows of w)."""
+    rc = _lib.lib().dz_gemm_skinny(
+        _lib.ptr(x2), ctypes.c_longlong(x2.stride(0)), _lib.ptr(w), ctypes.c_longlong(w.stride(0)),
+        _lib.ptr(out2), ctypes.c_longlong(out2.stride(0)), _lib.ptr(bias), _lib.ptr(res2),
+        ctypes.c_longlong(res2.stride(0) if res2 is not None else 0), x2.shape[0], out2.shape[1], x2.shape[1], act,
+        int(out2.dtype == torch.float32), ctypes.c_float(scale), splits, _lib.ptr(_lib.err_word(x2.device)),
+        _lib.stream_ptr())
+    _lib.check(rc, "dz_gemm_skinny")
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, act: str | None = None,
            residual: torch.Tensor | None = None, scale: float = 1.0,
            out_dtype: torch.dtype | None = None, out: torch.Tensor | None = None,
@@ -132,6 +160,9 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, a
     if M == 0:
         return out.reshape(*x.shape[:-1], N)
     variant = _VARIANT
+    if variant == 0 and tile_n == 0 and _skinny_pays(M, N):
+        _skinny(x2, w, out2, bias, res2, ACT[act], scale)
+        return out.reshape(*x.shape[:-1], N)
     if tile_n == 512:
         variant, tile_n = 2, 0
     elif tile_n in (128, 256):
