@@ -47,16 +47,39 @@ def filter_logits(logits: torch.Tensor, temperature: float = 1.0, top_k: Optiona
 
 
 class _Decoder:
-    """Per-layer K/V caches and the single-token step."""
+    """Per-layer K/V caches and the single-token step.
+
+    On CUDA every block of a step is launched by one native call (:class:`dizo_b200.ops.decode.DecodePlan`, built at the
+    first step of a run); CPU tensors, more than ``MAX_STEP_ROWS`` sequences and LoRA operands that share one merge buffer
+    go block by block through ``model.decode_block``."""
 
     def __init__(self, model: OPTModel, B: int, max_len: int):
         self.m = model
         cfg = model.config
         d = cfg.hidden_size
         dev, dt = model.device, model.dtype
-        self.k = [torch.zeros(B, max_len, d, dtype=dt, device=dev) for _ in range(cfg.num_hidden_layers)]
-        self.v = [torch.zeros(B, max_len, d, dtype=dt, device=dev) for _ in range(cfg.num_hidden_layers)]
+        # columns are written before they are read: no initial value
+        kv = torch.empty(2 * cfg.num_hidden_layers, B, max_len, d, dtype=dt, device=dev)
+        self.k, self.v = list(kv[0::2]), list(kv[1::2])
         self.len = 0
+        self.plan, self._caches = None, None
+        self.native = (dev.type == "cuda" and dt == torch.bfloat16 and B <= decode_ops.MAX_STEP_ROWS
+                       and getattr(type(model), "step_layer", None) is not None)
+
+    def _build_plan(self) -> None:
+        m, cfg = self.m, self.m.config
+        layers = []
+        for i in range(cfg.num_hidden_layers):
+            layers.append(m.step_layer(m._layer_weights(i, m._resolver(i, None, None, 0))))
+            if m.use_lora and not m._merge_buf["per_layer"]:
+                self.native = False                            # one merge buffer for all blocks: merged anew per block
+                return
+        if not layers:
+            self.native = False
+            return
+        B, max_len, d = self.k[0].shape
+        self.plan = decode_ops.DecodePlan(layers, B=B, d=d, ld_seq=max_len * d, ld_row=d,
+                                          **m.step_config(m.num_prefix + max_len))
 
     def prefill(self, batch: Batch) -> torch.Tensor:
         m = self.m
@@ -81,12 +104,21 @@ class _Decoder:
         for i in range(len(self.k)):
             self.k[i] = self.k[i].index_select(0, index)
             self.v[i] = self.v[i].index_select(0, index)
+        self._caches = None
 
     def step(self, tokens: torch.Tensor, positions: torch.Tensor, pad_left: torch.Tensor) -> torch.Tensor:
         """tokens, positions: int32 [B]; returns the next-token logits [B, V] (fp32)."""
         m = self.m
         t = self.len
         h = m.decode_embed(tokens, positions, m._resolver(-1, None, None, 0))
+        if self.native and self.plan is None:
+            self._build_plan()
+        if self.native:
+            if self._caches is None:
+                self._caches = self.plan.caches(self.k, self.v)
+            self.plan.h.copy_(h)
+            self.len = t + 1
+            return _head_logits(m, self.plan.step(self._caches, t, pad_left))
         for i in range(m.config.num_hidden_layers):
             w = m._layer_weights(i, m._resolver(i, None, None, 0))
             h = m.decode_block(h, w, self.k[i], self.v[i], t, pad_left)
@@ -291,6 +323,33 @@ def _make_decoder(model, B: int, max_len: int) -> _Decoder:
     raise NotImplementedError(f"autoregressive decoding is not built for {kind}")
 
 
+def _extend(dec: _Decoder, logits: torch.Tensor, out: List[List[int]], pos: torch.Tensor, pad_left: torch.Tensor,
+            max_new_tokens: int, eos: set, pad_token_id: int, **sampling) -> None:
+    """Greedy / sampled continuation of the rows of ``out`` on CUDA.  A token stays on the device between the sampling
+    kernel and the next step, which is queued before the host looks at the token: the host's part runs beside the step."""
+    dev = logits.device
+    B = len(out)
+    done = torch.zeros(B, dtype=torch.int32, device=dev)
+    eos_dev = torch.tensor(sorted(eos), dtype=torch.int32).to(dev) if eos else None
+    host = torch.empty((max_new_tokens, B), dtype=torch.int32, pin_memory=True)
+    ended = [False] * B
+    ready = torch.cuda.Event()
+    for t in range(max_new_tokens):
+        nxt = decode_ops.sample_step(logits, offset=t, done=done, eos=eos_dev, pad_id=pad_token_id, **sampling)
+        host[t].copy_(nxt, non_blocking=True)
+        ready.record()
+        if t + 1 < max_new_tokens:
+            logits = dec.step(nxt, pos, pad_left)
+            pos = pos + 1
+        ready.synchronize()
+        for i, tok in enumerate(host[t].tolist()):
+            if not ended[i]:
+                out[i].append(tok)
+                ended[i] = tok in eos
+        if all(ended):
+            break
+
+
 @torch.no_grad()
 def generate(model: OPTModel, input_ids: torch.Tensor, attention_mask: Optional[torch.Tensor] = None,
              max_new_tokens: int = 50, do_sample: bool = False, temperature: float = 1.0,
@@ -321,6 +380,10 @@ def generate(model: OPTModel, input_ids: torch.Tensor, attention_mask: Optional[
     if seed is not None:
         gen.manual_seed(seed)
     out = [row[m.bool()].tolist() for row, m in zip(ids, mask)]
+    if nb == 1 and type(dec) is _Decoder and dev.type == "cuda":
+        _extend(dec, logits, out, (n_real + 2).to(torch.int32), pad_left, max_new_tokens, eos, pad_token_id,
+                temperature=temperature, top_k=top_k, top_p=top_p, do_sample=do_sample, seed=seed or 0)
+        return out
     done = torch.zeros(B, dtype=torch.bool, device=dev)
     beam_score = torch.zeros(B, device=dev)
     if nb > 1:

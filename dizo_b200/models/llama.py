@@ -279,3 +279,14 @@ class LlamaModel(OPTModel):
                                           w.prefix_k, w.prefix_v)
         h = gemm.linear(ctx.contiguous(), w.out_w, residual=h)
         return self._mlp(h, w)
+
+    @staticmethod
+    def step_layer(w: SimpleNamespace) -> dict:
+        return dict(ln1_w=w.ln1_w, qkv_w=w.qkv_w, out_w=w.out_w, ln2_w=w.ln2_w, up_w=w.gu_w, down_w=w.down_w,
+                    prefix_k=w.prefix_k, prefix_v=w.prefix_v)
+
+    def step_config(self, n_pos: int) -> dict:
+        cfg = self.config
+        return dict(F=cfg.ffn_dim, H=cfg.num_attention_heads, Hkv=cfg.num_key_value_heads, act=3, rms=True,
+                    pre_norm=True, eps=cfg.rms_norm_eps,
+                    rope=llama_ops.rope_table(n_pos, cfg.head_dim, cfg.rope_theta, self.device))

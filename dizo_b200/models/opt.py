@@ -743,6 +743,20 @@ class OPTModel:
             h = norm.layernorm(h, w.ln2_w, w.ln2_b, cfg.layer_norm_eps)
         return h
 
+    @staticmethod
+    def step_layer(w: SimpleNamespace) -> dict:
+        """One block's weights under the names of ``ops.decode.DecodePlan``."""
+        return dict(ln1_w=w.ln1_w, ln1_b=w.ln1_b, qkv_w=w.qkv_w, qkv_b=w.qkv_b, out_w=w.out_w, out_b=w.out_b,
+                    ln2_w=w.ln2_w, ln2_b=w.ln2_b, up_w=w.fc1_w, up_b=w.fc1_b, down_w=w.fc2_w, down_b=w.fc2_b,
+                    prefix_k=w.prefix_k, prefix_v=w.prefix_v)
+
+    def step_config(self, n_pos: int) -> dict:
+        """What a ``DecodePlan`` for positions below ``n_pos`` needs beside the weights."""
+        cfg = self.config
+        return dict(F=cfg.ffn_dim, H=cfg.num_attention_heads, Hkv=cfg.num_attention_heads,
+                    act=gemm.ACT[cfg.activation_function], rms=False, pre_norm=cfg.do_layer_norm_before,
+                    eps=cfg.layer_norm_eps)
+
     def _selected(self, batch: Batch, transform: Transform | None) -> torch.Tensor:
         """Final-normalised hidden rows ``batch.rows``.  The replicated model restricts its last block to
         them; sharded layouts (own ``hidden_states``) compute every row and pick afterwards."""

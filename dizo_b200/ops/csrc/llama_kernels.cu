@@ -12,6 +12,8 @@
 // silu_mul: out[m, f] = silu(gu[m, f]) * gu[m, F + f] for the fused gate | up projection output.
 #include "common.cuh"
 #include "host_util.h"
+#include "norm.h"
+#include "pdl.cuh"
 
 namespace dz {
 
@@ -22,6 +24,8 @@ __global__ void __launch_bounds__(THREADS)
 rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
                __nv_bfloat16* __restrict__ y, long long ldy, int d, float eps) {
   __shared__ float s_red[THREADS / 32];
+  pdl_trigger();
+  pdl_wait();
   const long long row = blockIdx.x;
   const int nvec = d >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * ldx);
@@ -121,6 +125,18 @@ silu_mul_kernel(const __nv_bfloat16* __restrict__ gu, long long ld, __nv_bfloat1
   }
 }
 
+int rmsnorm_launch(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, __nv_bfloat16* y, long long ldy,
+                   long long rows, int d, float eps, bool dependent, cudaStream_t stream) {
+  const int nvec = d >> 3;
+  auto launch = [&](auto kern, int threads) {
+    return cuda_rc(pdl_launch(kern, dim3((unsigned)rows), threads, 0, stream, 1, dependent, x, ldx, w, y, ldy, d, eps));
+  };
+  if (nvec <= 128 * RMS_MAXV) return launch(rmsnorm_kernel<128>, 128);
+  if (nvec <= 256 * RMS_MAXV) return launch(rmsnorm_kernel<256>, 256);
+  if (nvec <= 512 * RMS_MAXV) return launch(rmsnorm_kernel<512>, 512);
+  return DZ_ERR_TOO_LARGE;
+}
+
 static inline bool lk_al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace dz
@@ -132,17 +148,8 @@ extern "C" int dz_rmsnorm(const void* x, long long ldx, const void* w, void* y, 
                           int d, float eps, cudaStream_t stream) {
   if (!x || !w || !y || rows <= 0 || d <= 0) return DZ_ERR_ARG;
   if ((d & 7) || (ldx & 7) || (ldy & 7) || !lk_al16(x) || !lk_al16(w) || !lk_al16(y)) return DZ_ERR_ALIGN;
-  const int nvec = d >> 3;
-  auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w; auto Y = (__nv_bfloat16*)y;
-  if (nvec <= 128 * RMS_MAXV)
-    rmsnorm_kernel<128><<<(unsigned)rows, 128, 0, stream>>>(X, ldx, W, Y, ldy, d, eps);
-  else if (nvec <= 256 * RMS_MAXV)
-    rmsnorm_kernel<256><<<(unsigned)rows, 256, 0, stream>>>(X, ldx, W, Y, ldy, d, eps);
-  else if (nvec <= 512 * RMS_MAXV)
-    rmsnorm_kernel<512><<<(unsigned)rows, 512, 0, stream>>>(X, ldx, W, Y, ldy, d, eps);
-  else
-    return DZ_ERR_TOO_LARGE;
-  return cuda_rc(cudaGetLastError());
+  return rmsnorm_launch((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, ldy, rows, d, eps,
+                        false, stream);
 }
 
 // in: bf16 [rows, ld_in] holding q (H*hd) | k (Hkv*hd) | v (Hkv*hd); out: bf16 [rows, ld_out] holding

@@ -10,6 +10,8 @@
 // :639, :657).
 #include "common.cuh"
 #include "host_util.h"
+#include "norm.h"
+#include "pdl.cuh"
 
 namespace dz {
 
@@ -22,6 +24,8 @@ layernorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
                  __nv_bfloat16* __restrict__ y, long long ldy, int d, float eps) {
   __shared__ float s_red[THREADS / 32];
   __shared__ float s_bcast;
+  pdl_trigger();
+  pdl_wait();
   const long long row = blockIdx.x;
   const int nvec = d >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * ldx);
@@ -152,6 +156,19 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ src, long long lds, const i
     if (DZ_STORE_OK(orow + i, 16)) orow[i] = sr[i];
 }
 
+int layernorm_launch(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* b,
+                     __nv_bfloat16* y, long long ldy, long long rows, int d, float eps, bool dependent,
+                     cudaStream_t stream) {
+  const int nvec = d >> 3;
+  auto launch = [&](auto kern, int threads) {
+    return cuda_rc(pdl_launch(kern, dim3((unsigned)rows), threads, 0, stream, 1, dependent, x, ldx, w, b, y, ldy, d, eps));
+  };
+  if (nvec <= 128 * LN_MAXV) return launch(layernorm_kernel<128>, 128);
+  if (nvec <= 256 * LN_MAXV) return launch(layernorm_kernel<256>, 256);
+  if (nvec <= 512 * LN_MAXV) return launch(layernorm_kernel<512>, 512);
+  return DZ_ERR_TOO_LARGE;
+}
+
 }  // namespace dz
 
 using namespace dz;
@@ -164,18 +181,8 @@ extern "C" int dz_layernorm(const void* x, long long ldx, const void* w, const v
   if (!x || !w || !b || !y || rows <= 0 || d <= 0) return DZ_ERR_ARG;
   if ((d & 7) || (ldx & 7) || (ldy & 7) || !al16(x) || !al16(w) || !al16(b) || !al16(y))
     return DZ_ERR_ALIGN;
-  const int nvec = d >> 3;
-  auto X = (const __nv_bfloat16*)x; auto W = (const __nv_bfloat16*)w;
-  auto Bb = (const __nv_bfloat16*)b; auto Y = (__nv_bfloat16*)y;
-  if (nvec <= 128 * LN_MAXV)
-    layernorm_kernel<128><<<(unsigned)rows, 128, 0, stream>>>(X, ldx, W, Bb, Y, ldy, d, eps);
-  else if (nvec <= 256 * LN_MAXV)
-    layernorm_kernel<256><<<(unsigned)rows, 256, 0, stream>>>(X, ldx, W, Bb, Y, ldy, d, eps);
-  else if (nvec <= 512 * LN_MAXV)
-    layernorm_kernel<512><<<(unsigned)rows, 512, 0, stream>>>(X, ldx, W, Bb, Y, ldy, d, eps);
-  else
-    return DZ_ERR_TOO_LARGE;
-  return cuda_rc(cudaGetLastError());
+  return layernorm_launch((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b,
+                          (__nv_bfloat16*)y, ldy, rows, d, eps, false, stream);
 }
 
 extern "C" int dz_embed(const int* ids, const int* positions, const void* tok, long long ld_tok,

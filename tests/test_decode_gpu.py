@@ -1,0 +1,91 @@
+"""Decoding kernels: native decoding steps against the block-by-block path, the sampler's two forms."""
+import pytest
+import torch
+
+from dizo_b200.models.generate import _Decoder
+from dizo_b200.models.llama import LlamaConfig, LlamaModel
+from dizo_b200.models.opt import OPTConfig, OPTModel, make_batch
+from dizo_b200.ops import _lib
+from dizo_b200.ops import decode as decode_ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _models():
+    opt = dict(vocab_size=520, hidden_size=160, num_hidden_layers=3, ffn_dim=328, max_position_embeddings=256)
+    lla = dict(vocab_size=520, hidden_size=512, num_hidden_layers=2, intermediate_size=712, max_position_embeddings=256)
+    return {
+        "opt": lambda: OPTModel(OPTConfig(num_attention_heads=2, **opt), "cuda", torch.bfloat16),
+        "opt-post": lambda: OPTModel(OPTConfig(num_attention_heads=10, do_layer_norm_before=False, word_embed_proj_dim=64,
+                                               **opt), "cuda", torch.bfloat16),
+        "opt-adapters": lambda: OPTModel(OPTConfig(num_attention_heads=2, **opt), "cuda", torch.bfloat16,
+                                         mode="lora+prefix"),
+        "llama": lambda: LlamaModel(LlamaConfig(num_attention_heads=4, num_key_value_heads=2, **lla), "cuda",
+                                    torch.bfloat16),
+        "llama-prefix": lambda: LlamaModel(LlamaConfig(num_attention_heads=16, num_key_value_heads=16, **lla), "cuda",
+                                           torch.bfloat16, mode="prefix"),
+    }
+
+
+@pytest.mark.parametrize("name", ["opt", "opt-post", "opt-adapters", "llama", "llama-prefix"])
+@pytest.mark.parametrize("B,L", [(1, 3), (5, 130), (40, 17)])
+def test_native_step_equals_block_by_block(name, B, L):
+    m = _models()[name]().init_random_fast(3, std=0.05)
+    for n in m.trainable_names:
+        if "lora_B" in n:
+            m.param(n).normal_(0, 0.05)
+    g = torch.Generator().manual_seed(B * L)
+    ids = torch.randint(4, 500, (B, L), generator=g)
+    mask = torch.ones_like(ids)
+    for i in range(1, B):
+        mask[i, :min(i, L - 1)] = 0
+    batch = make_batch(ids, mask).to("cuda")
+    decs = [_Decoder(m, B, L + 8) for _ in range(2)]
+    assert decs[0].native
+    decs[1].native = False
+    first = [d.prefill(batch) for d in decs]
+    assert torch.equal(first[0], first[1])
+    pos = (mask.sum(1).cuda() + 2).to(torch.int32)
+    for t in range(3):
+        tok = torch.full((B,), 7 + t, dtype=torch.int32, device="cuda")
+        a, b = (d.step(tok, pos + t, batch.pad_left) for d in decs)
+        _lib.check_device_errors()
+        # the same kernels on the same operands: K / V append and attention sum the same keys, with the newest key taken
+        # from registers instead of the cache (another order of fp32 sums); LLaMA's SwiGLU is the same launch
+        assert ((a - b).norm() / b.norm()).item() < 2 * 2.0 ** -8
+        for x, y in zip(decs[0].k + decs[0].v, decs[1].k + decs[1].v):
+            x, y = x[:, :L + t + 1].float(), y[:, :L + t + 1].float()
+            assert ((x - y).norm() / y.norm()).item() < 2 * 2.0 ** -8
+    index = torch.arange(B - 1, -1, -1, device="cuda")
+    for d in decs:
+        d.reorder(index)
+    a, b = (d.step(tok, pos + 3, batch.pad_left[index]) for d in decs)
+    assert ((a - b).norm() / b.norm()).item() < 2 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("V", [7, 512, 2049, 32000, 51200])
+@pytest.mark.parametrize("top_k,top_p", [(None, None), (40, None), (None, 0.9), (300, 0.6)])
+def test_sampler_forms_agree(V, top_k, top_p):
+    """The shared-memory form and the form for vocabularies beyond it draw the same tokens: columns of -inf that push the
+    row over the limit add exact zeros to every sum."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = torch.randn(6, V, device="cuda", generator=g) * 3
+    logits[5] = 0.0
+    wide = torch.full((6, 51300), float("-inf"), device="cuda")
+    wide[:, :V] = logits
+    for off in range(4):
+        a = decode_ops.sample(logits, 0.8, top_k, top_p, True, seed=11, offset=off)
+        b = decode_ops.sample(wide, 0.8, top_k, top_p, True, seed=11, offset=off)
+        assert torch.equal(a, b)
+        p = torch.softmax(logits / 0.8, -1)
+        assert (p.gather(1, a[:, None]) > 0).all()
+    assert torch.equal(decode_ops.sample(logits, do_sample=False), logits.argmax(-1))
+
+
+def test_sample_step_marks_finished_rows():
+    logits = torch.full((3, 100), -5.0, device="cuda")
+    logits[0, 9], logits[1, 4], logits[2, 50] = 5.0, 5.0, 5.0
+    done = torch.tensor([0, 0, 1], dtype=torch.int32, device="cuda")
+    eos = torch.tensor([4, 60], dtype=torch.int32, device="cuda")
+    out = decode_ops.sample_step(logits, do_sample=False, done=done, eos=eos, pad_id=1)
+    assert out.tolist() == [9, 4, 1] and done.tolist() == [0, 1, 1]
