@@ -5,7 +5,7 @@ over a deep copy of the model (large_models/trainer.py:714-741, :805-830).  Only
 are needed for that (no weight gradient is ever materialised: d loss / d alpha of a constrained
 tensor W_eff = theta_0 + alpha (theta - theta_0) is the contraction <dY, X (theta - theta_0)^T>),
 so the set is: the data-gradient GEMM dX = dY W with the weight read in place as the MN-major
-tcgen05 operand (``csrc/gemm_sm100.cu``), the attention backward (``csrc/attn_bwd_sm100.cu``,
+tcgen05 operand (``csrc/gemm2_sm100.cu``, small ones ``csrc/gemm_sm100.cu``), the attention backward (``csrc/attn_bwd_sm100.cu``,
 bound in :mod:`dizo_b200.ops.attention`) and the memory-bound pieces of ``csrc/bwd_kernels.cu``.
 CPU tensors run the plain PyTorch statement of each op (the oracle of the GPU tests).
 """
@@ -43,7 +43,10 @@ def linear_dgrad(dy: torch.Tensor, w: torch.Tensor, mask: torch.Tensor | None = 
         assert mask.dtype == torch.bfloat16 and mask.shape == (M, N) and mask.stride(1) == 1
     if residual is not None:
         assert residual.dtype == torch.bfloat16 and residual.shape == (M, N) and residual.stride(1) == 1
-    rc = _lib.lib().dz_gemm_bf16_nn(
+    # pairs of SMs (256-row tiles) under the rule of ``gemm.linear``
+    pair = M >= 256 and ((M + 255) // 256) * ((N + 255) // 256) >= 48
+    f = _lib.lib().dz_gemm2_bf16_nn if pair else _lib.lib().dz_gemm_bf16_nn
+    rc = f(
         _lib.ptr(dy), ll(dy.stride(0)), _lib.ptr(w), ll(w.stride(0)), _lib.ptr(out), ll(out.stride(0)),
         _lib.ptr(residual), ll(residual.stride(0) if residual is not None else 0),
         _lib.ptr(mask), ll(mask.stride(0) if mask is not None else 0), M, N, K,

@@ -38,11 +38,14 @@ constexpr uint32_t G2_TMEM_COLS = 2 * G2_BN;
 struct Gemm2Args {
   int M, N, K;
   int num_m, num_n, group_m;
+  int bn;                   // columns of a tile
   void* out;
   long long ldo;
   const __nv_bfloat16* bias;
   const __nv_bfloat16* residual;
   long long ldr;
+  const __nv_bfloat16* mask;      // [M, ldm] or null: the result is zeroed where mask <= 0 (ReLU backward)
+  long long ldm;
   int act;
   int out_fp32;
   float out_scale;
@@ -50,6 +53,7 @@ struct Gemm2Args {
   // act 4: rotary embedding of a fused q | k | v projection in the epilogue (head dim 128)
   int wide_store;           // out and its row pitch are 32-byte aligned: 256-bit stores in the bf16 epilogues
   int wide_residual;        // the same for the residual rows: 256-bit loads
+  int wide_mask;            // the mask rows are 16-byte aligned
   const float* rope_cs;     // fp32 [n_pos][64][2] = (cos, sin)
   int rope_L, rope_pos0, rope_n_pos, rope_H, rope_Hkv;
 };
@@ -64,8 +68,14 @@ __device__ __forceinline__ void tile_coords2(int tile, const Gemm2Args& p, int& 
   nb = r / gm;
 }
 
+// B_MN = false: W is [N, K] row-major (out = A W^T, both operands K-major).
+// B_MN = true : W is [K, N] row-major (out = A W, the data gradient of a linear layer): the B operand is MN-major, each CTA
+//               stages its half of the columns as 64-column panels of [64 k-rows][128 B].  With the ReLU mask, one-SM
+//               kernel (gemm_sm100.cu) and this one, us: M 4096 N 10240 K 2560 383 and 148 (the one-SM epilogue also reads
+//               the mask two bytes at a time), M 4096 N 2560 K 10240 239 and 187, M 8192 N 5120 K 5120 428 and 284.
+template <bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2_THREADS, 1)
-gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const Gemm2Args p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[G2_STAGES];    // used in the leader only
@@ -127,13 +137,19 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           const uint32_t full_leader = map_to_cta(full_local, 0);
           const uint32_t a_dst = smem_base + stage * G2_STAGE_BYTES;
           const uint32_t b_dst = a_dst + G2_A_BYTES;
-          if (leader) mbar_arrive_expect_tx(full_local, 2 * G2_STAGE_BYTES);  // both CTAs' bytes
+          if (leader)                                                         // both CTAs' bytes
+            mbar_arrive_expect_tx(full_local, 2 * G2_A_BYTES + p.bn * (G2_BK * 2));
           tma_load_2d_2sm(a_dst, &tmA, full_leader, kb * G2_BK, mb * G2_BM + (int)rank * 128);
           // act 3 (SwiGLU over W = gate rows | up rows): the leader's half of the tile is 128 gate rows, the
           // peer's half the matching 128 up rows, so that column j and column 128 + j of the accumulator pair up
           const int b_row = p.act == 3 ? (int)rank * (p.N >> 1) + nb * (G2_BN / 2)
-                                       : nb * G2_BN + (int)rank * (G2_BN / 2);
-          tma_load_2d_2sm(b_dst, &tmB, full_leader, kb * G2_BK, b_row);
+                                       : nb * p.bn + (int)rank * (p.bn >> 1);
+          if (B_MN) {
+            for (int c = 0; c < p.bn / 128; ++c)
+              tma_load_2d_2sm(b_dst + c * (G2_BK * 128), &tmB, full_leader, b_row + c * 64, kb * G2_BK);
+          } else {
+            tma_load_2d_2sm(b_dst, &tmB, full_leader, kb * G2_BK, b_row);
+          }
           if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -141,7 +157,7 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA)
     if (leader && elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(G2_BM, G2_BN);
+      const uint32_t idesc = umma_idesc_bf16(G2_BM, p.bn, 0, B_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -164,10 +180,12 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           const uint32_t a_src = smem_base + stage * G2_STAGE_BYTES;
           const uint32_t b_src = a_src + G2_A_BYTES;
           const uint64_t a_desc = umma_desc_k_sw128(a_src);
-          const uint64_t b_desc = umma_desc_k_sw128(b_src);
+          // 16 K steps on: 32 bytes inside the swizzle row (K-major), two 8-row groups of 1024 bytes (MN-major)
+          const uint64_t b_desc = B_MN ? umma_desc_mn_sw128(b_src, G2_BK * 128, 1024) : umma_desc_k_sw128(b_src);
+          constexpr uint64_t b_step = B_MN ? (2048 >> 4) : 2;
 #pragma unroll
           for (int k = 0; k < G2_BK / 16; ++k)
-            umma_bf16_ss_2sm(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb | k) != 0);
+            umma_bf16_ss_2sm(d_tmem, a_desc + 2 * k, b_desc + b_step * k, idesc, (kb | k) != 0);
           umma_commit_2sm(smem_u32(&bar_empty[stage]), 3);     // frees the stage in both CTAs
           if (++stage == G2_STAGES) { stage = 0; phase ^= 1; }
         }
@@ -272,11 +290,11 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
       } else {
 #pragma unroll 1
-      for (int c = 0; c < G2_BN / 32; ++c) {
+      for (int c = 0; c < p.bn / 32; ++c) {
         uint32_t r[32];
         tmem_ld_32x32(t_row + c * 32, r);
         tmem_ld_wait();
-        const int col0 = nb * G2_BN + c * 32;
+        const int col0 = nb * p.bn + c * 32;
         if (col0 >= p.N) continue;
         float v[32];
 #pragma unroll
@@ -311,6 +329,25 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
         }
         if (row_ok) {
+          if (B_MN && p.mask) {
+            const __nv_bfloat16* mp = p.mask + row * p.ldm + col0;
+            if (full_chunk && p.wide_mask) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const uint4 b = __ldg(reinterpret_cast<const uint4*>(mp) + q);
+                const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  if (!(bf16_lo(w[j]) > 0.f)) v[q * 8 + 2 * j] = 0.f;
+                  if (!(bf16_hi(w[j]) > 0.f)) v[q * 8 + 2 * j + 1] = 0.f;
+                }
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (col0 + j < p.N && !(__bfloat162float(mp[j]) > 0.f)) v[j] = 0.f;
+            }
+          }
           if (p.residual) {
             const __nv_bfloat16* rp = p.residual + row * p.ldr + col0;
             if (full_chunk && p.wide_residual) {
@@ -404,10 +441,18 @@ gemm2_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 using namespace dz;
 DZ_DEBUG_TU(gemm2)
 
+// What a launch adds to the plain product.
+struct Gemm2Extra {
+  const void* mask;         // ReLU backward (MN-major form)
+  long long ldm;
+  const Gemm2Args* rope;    // act 4
+};
+
+template <bool B_MN>
 static int gemm2_launch(const void* A, long long lda, const void* W, long long ldw, void* out,
                         long long ldo, const void* bias, const void* residual, long long ldr,
                         int M, int N, int K, int act, int out_fp32, float out_scale,
-                        uint32_t* err, cudaStream_t stream, const Gemm2Args* rope);
+                        uint32_t* err, cudaStream_t stream, const Gemm2Extra& extra);
 
 // Same contract as dz_gemm_bf16_tn (gemm_sm100.cu); computed by pairs of SMs.
 extern "C" int dz_gemm2_bf16_tn(const void* A, long long lda, const void* W, long long ldw, void* out,
@@ -415,8 +460,19 @@ extern "C" int dz_gemm2_bf16_tn(const void* A, long long lda, const void* W, lon
                                 int M, int N, int K, int act, int out_fp32, float out_scale,
                                 uint32_t* err, cudaStream_t stream) {
   if (act == 4) return DZ_ERR_ARG;
-  return gemm2_launch(A, lda, W, ldw, out, ldo, bias, residual, ldr, M, N, K, act, out_fp32, out_scale, err,
-                      stream, nullptr);
+  return gemm2_launch<false>(A, lda, W, ldw, out, ldo, bias, residual, ldr, M, N, K, act, out_fp32, out_scale, err,
+                             stream, Gemm2Extra{});
+}
+
+// Same contract as dz_gemm_bf16_nn (gemm_sm100.cu): out = (A W) masked + residual with W [K, N] row-major.
+extern "C" int dz_gemm2_bf16_nn(const void* A, long long lda, const void* W, long long ldw, void* out,
+                                long long ldo, const void* residual, long long ldr, const void* mask,
+                                long long ldm, int M, int N, int K, int out_fp32, uint32_t* err,
+                                cudaStream_t stream) {
+  if (N & 7) return DZ_ERR_ALIGN;
+  Gemm2Extra x{};
+  x.mask = mask; x.ldm = ldm;
+  return gemm2_launch<true>(A, lda, W, ldw, out, ldo, nullptr, residual, ldr, M, N, K, 0, out_fp32, 1.0f, err, stream, x);
 }
 
 // Fused q | k | v projection with the rotary embedding in the epilogue: A [M, K], W [(H + 2 Hkv) * 128, K] ->
@@ -430,14 +486,17 @@ extern "C" int dz_gemm2_qkv_rope(const void* A, long long lda, const void* W, lo
   if (ldo < 3LL * H * 128 || (reinterpret_cast<uintptr_t>(cs) & 15)) return DZ_ERR_ALIGN;
   Gemm2Args r{};
   r.rope_cs = cs; r.rope_L = L; r.rope_pos0 = pos0; r.rope_n_pos = n_pos; r.rope_H = H; r.rope_Hkv = Hkv;
-  return gemm2_launch(A, lda, W, ldw, out, ldo, nullptr, nullptr, 0, M, (H + 2 * Hkv) * 128, K, 4, 0, 1.0f, err,
-                      stream, &r);
+  Gemm2Extra x{};
+  x.rope = &r;
+  return gemm2_launch<false>(A, lda, W, ldw, out, ldo, nullptr, nullptr, 0, M, (H + 2 * Hkv) * 128, K, 4, 0, 1.0f, err,
+                             stream, x);
 }
 
+template <bool B_MN>
 static int gemm2_launch(const void* A, long long lda, const void* W, long long ldw, void* out,
                         long long ldo, const void* bias, const void* residual, long long ldr,
                         int M, int N, int K, int act, int out_fp32, float out_scale,
-                        uint32_t* err, cudaStream_t stream, const Gemm2Args* rope) {
+                        uint32_t* err, cudaStream_t stream, const Gemm2Extra& extra) {
   if (!A || !W || !out || M <= 0 || N <= 0 || K <= 0) return DZ_ERR_ARG;
   if ((K & 7) || (lda & 7) || (ldw & 7)) return DZ_ERR_ALIGN;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return DZ_ERR_ALIGN;
@@ -458,28 +517,14 @@ static int gemm2_launch(const void* A, long long lda, const void* W, long long l
   static const bool st256 = [] { const char* e = getenv("DIZO_GEMM_ST256"); return !(e && e[0] == '0'); }();
   a.wide_store = st256 && !out_fp32 && !(reinterpret_cast<uintptr_t>(out) & 31) && !(ldo & 15);
   a.wide_residual = st256 && residual && !(reinterpret_cast<uintptr_t>(residual) & 31) && !(ldr & 15);
-  if (rope) {
+  a.mask = reinterpret_cast<const __nv_bfloat16*>(extra.mask); a.ldm = extra.ldm;
+  a.wide_mask = extra.mask && !(reinterpret_cast<uintptr_t>(extra.mask) & 15) && !(extra.ldm & 7);
+  if (const Gemm2Args* rope = extra.rope) {
     a.rope_cs = rope->rope_cs; a.rope_L = rope->rope_L; a.rope_pos0 = rope->rope_pos0;
     a.rope_n_pos = rope->rope_n_pos; a.rope_H = rope->rope_H; a.rope_Hkv = rope->rope_Hkv;
   }
-  a.num_m = (M + G2_BM - 1) / G2_BM;
-  a.num_n = (N + G2_BN - 1) / G2_BN;
-  // M tiles per rasterisation group: a group's A tiles stay in L2 while its W tiles stream once
-  static const int group_env = [] { const char* e = getenv("DIZO_GEMM_GROUP_M"); return e ? atoi(e) : 0; }();
-  // 16 while the group's A tiles (256 x K bf16 each) stay within about 48 MB of L2 (K = 5120: +1 % over 8 on the
-  // QKV / fc1 / out_proj shapes), else 8 (K = 20480: 16 measured -0.8 %, 4 measured -5 %, 32 is worse everywhere);
-  // DIZO_GEMM_GROUP_M overrides for measurements
-  int gm = (long long)16 * G2_BM * K * 2 > (48LL << 20) ? 8 : 16;
-  if (group_env > 0) gm = group_env;
-  a.group_m = a.num_m < gm ? a.num_m : gm;
-  CUtensorMap tmA, tmB;
-  int rc = make_tmap_bf16_2d(&tmA, A, M, K, lda, 128, G2_BK, true);
-  if (rc) return rc;
-  rc = make_tmap_bf16_2d(&tmB, W, N, K, ldw, G2_BN / 2, G2_BK, true);
-  if (rc) return rc;
   static PerDeviceFlag configured;
-  if (int rc_cfg = ensure_dyn_smem(configured, gemm2_bf16_tn_kernel, G2_SMEM)) return rc_cfg;
-  int tiles = a.num_m * a.num_n;
+  if (int rc_cfg = ensure_dyn_smem(configured, gemm2_bf16_kernel<B_MN>, G2_SMEM)) return rc_cfg;
   static int max_clusters = 0;
   if (!max_clusters) {
     cudaLaunchConfig_t cfg = {};
@@ -492,14 +537,32 @@ static int gemm2_launch(const void* A, long long lda, const void* W, long long l
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_tn_kernel, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, gemm2_bf16_kernel<B_MN>, &cfg) != cudaSuccess || n <= 0) {
       (void)cudaGetLastError();
       n = sm_count() / 2;
     }
     max_clusters = n < sm_count() / 2 ? n : sm_count() / 2;
   }
+  a.num_m = (M + G2_BM - 1) / G2_BM;
+  a.bn = G2_BN;
+  a.num_n = (N + a.bn - 1) / a.bn;
+  // M tiles per rasterisation group: a group's A tiles stay in L2 while its W tiles stream once
+  static const int group_env = [] { const char* e = getenv("DIZO_GEMM_GROUP_M"); return e ? atoi(e) : 0; }();
+  // 16 while the group's A tiles (256 x K bf16 each) stay within about 48 MB of L2 (K = 5120: +1 % over 8 on the
+  // QKV / fc1 / out_proj shapes), else 8 (K = 20480: 16 measured -0.8 %, 4 measured -5 %, 32 is worse everywhere);
+  // DIZO_GEMM_GROUP_M overrides for measurements
+  int gm = (long long)16 * G2_BM * K * 2 > (48LL << 20) ? 8 : 16;
+  if (group_env > 0) gm = group_env;
+  a.group_m = a.num_m < gm ? a.num_m : gm;
+  CUtensorMap tmA, tmB;
+  int rc = make_tmap_bf16_2d(&tmA, A, M, K, lda, 128, G2_BK, true);
+  if (rc) return rc;
+  rc = B_MN ? make_tmap_bf16_2d(&tmB, W, K, N, ldw, G2_BK, 64, true)             // box: 64 k-rows x 64 columns
+            : make_tmap_bf16_2d(&tmB, W, N, K, ldw, a.bn / 2, G2_BK, true);
+  if (rc) return rc;
+  const int tiles = a.num_m * a.num_n;
   int clusters = max_clusters;
   if (tiles < clusters) clusters = tiles;
-  gemm2_bf16_tn_kernel<<<clusters * 2, G2_THREADS, G2_SMEM, stream>>>(tmA, tmB, a);
+  gemm2_bf16_kernel<B_MN><<<clusters * 2, G2_THREADS, G2_SMEM, stream>>>(tmA, tmB, a);
   return cuda_rc(cudaGetLastError());
 }

@@ -22,7 +22,7 @@ def _rel(a, b):
 
 
 @pytest.mark.parametrize("M,K,N", [(300, 512, 768), (1024, 2048, 1000), (64, 50272, 256), (130, 72, 264),
-                                   (2048, 1024, 4096)])
+                                   (2048, 1024, 4096), (1400, 72, 4088), (3000, 328, 1032)])
 def test_linear_dgrad(M, K, N):
     g = torch.Generator(device=DEV).manual_seed(M + K + N)
     dy = torch.randn(M, K, device=DEV, generator=g).bfloat16()
