@@ -38,7 +38,7 @@ constexpr uint32_t G2_TMEM_COLS = 2 * G2_BN;
 struct Gemm2Args {
   int M, N, K;
   int num_m, num_n, group_m;
-  int bn;                   // columns of a tile
+  int bn;                   // columns of a tile: 256 or 224 (the latter with the plain epilogue only)
   void* out;
   long long ldo;
   const __nv_bfloat16* bias;
@@ -454,6 +454,22 @@ static int gemm2_launch(const void* A, long long lda, const void* W, long long l
                         int M, int N, int K, int act, int out_fp32, float out_scale,
                         uint32_t* err, cudaStream_t stream, const Gemm2Extra& extra);
 
+// Width of a tile: 256, or 224 columns where that makes the last wave of tiles fuller.  A narrower tile costs more than its
+// share (the A operand is fetched as before): a wave of 224-column tiles was measured at 0.87-0.91 of a 256-column one over
+// K = 2048 to 20480 (192, 160 and 128 columns: 0.78, 0.73, 0.69, which gained nothing within a training step).  Taken from
+// 2 % up; below that the extra operand traffic costs more power than the wave saves (M 8192, N = K = 5120: 283 us at 256,
+// 292 at 224).  Measured, us at 256 and 224: M 4096 N 2560 K 10240 181 and 159, M 3000 N 2560 K 2560 36.2 and 32.8, M 1920
+// N 8192 K 2048 55.5 and 49.9 (each the same number of waves of smaller tiles); the gamma search of OPT-2.7b, 16 x 256
+// tokens, 415 -> 408 ms.
+static int gemm2_tile_n(int num_m, int N, int clusters) {
+  constexpr int narrow = 224;
+  auto waves = [&](int bn) {
+    const long long tiles = (long long)num_m * ((N + bn - 1) / bn);
+    return (float)((tiles + clusters - 1) / clusters);
+  };
+  return 0.89f * waves(narrow) < 0.98f * waves(G2_BN) ? narrow : G2_BN;
+}
+
 // Same contract as dz_gemm_bf16_tn (gemm_sm100.cu); computed by pairs of SMs.
 extern "C" int dz_gemm2_bf16_tn(const void* A, long long lda, const void* W, long long ldw, void* out,
                                 long long ldo, const void* bias, const void* residual, long long ldr,
@@ -544,7 +560,7 @@ static int gemm2_launch(const void* A, long long lda, const void* W, long long l
     max_clusters = n < sm_count() / 2 ? n : sm_count() / 2;
   }
   a.num_m = (M + G2_BM - 1) / G2_BM;
-  a.bn = G2_BN;
+  a.bn = act >= 3 || B_MN ? G2_BN : gemm2_tile_n(a.num_m, N, max_clusters);
   a.num_n = (N + a.bn - 1) / a.bn;
   // M tiles per rasterisation group: a group's A tiles stay in L2 while its W tiles stream once
   static const int group_env = [] { const char* e = getenv("DIZO_GEMM_GROUP_M"); return e ? atoi(e) : 0; }();

@@ -67,3 +67,22 @@ def test_gemm_deterministic():
         a = linear(x, w, tile_n=tn)
         b = linear(x, w, tile_n=tn)
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M,N,K", [(4096, 2560, 136), (4032, 4096, 72), (1920, 8192, 64), (3000, 2560, 328),
+                                   (3000, 2552, 200), (4032, 4088, 136)])
+def test_two_sm_tile_widths(M, N, K):
+    """Shapes around the choice of 224-column tiles (last wave of 256-column tiles nearly empty), with ragged edges: the sums
+    run over the same K blocks in the same order as the one-SM kernel's, so the results are equal."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.05).bfloat16()
+    b = torch.randn(N, device="cuda", generator=g).bfloat16()
+    r = torch.randn(M, N, device="cuda", generator=g).bfloat16()
+    for dtype in (torch.bfloat16, torch.float32):
+        y = linear(x, w, b, act="relu", residual=r, out_dtype=dtype, tile_n=512)
+        z = linear(x, w, b, act="relu", residual=r, out_dtype=dtype, tile_n=256)
+        _lib.check_device_errors()
+        assert torch.equal(y, z)
+        ref = linear_reference(x, w, b, act="relu", residual=r, out_dtype=torch.float32)
+        assert _rel_err(y, ref) < (1e-4 if dtype == torch.float32 else 6e-3)
