@@ -72,6 +72,44 @@ __device__ __forceinline__ Philox4 z_words(uint64_t seed, uint32_t tid, uint32_t
                                      static_cast<uint32_t>(seed >> 32));
 }
 
+// What the first two rounds of a tensor's stream have in common for every group: counter (grp, tid, stream, 0) puts the
+// uniform words (tid, stream) through the first round alone, and the first product of the second round is uniform too.
+// Held per tensor, they take two of the fourteen wide multiplies and their key arithmetic out of every call.
+struct PhiloxStream {
+  uint32_t k0, k1;        // key
+  uint32_t p_hi, p_lo;    // M0 * (first word after round 1)
+  uint32_t x;             // low product of the stream word, xor the second round's first key word
+};
+__device__ __forceinline__ PhiloxStream philox_stream(uint64_t seed, uint32_t tid, uint32_t stream) {
+  PhiloxStream s;
+  s.k0 = static_cast<uint32_t>(seed);
+  s.k1 = static_cast<uint32_t>(seed >> 32);
+  const uint64_t p1 = static_cast<uint64_t>(PHILOX_M1) * stream;
+  const uint64_t p0 = static_cast<uint64_t>(PHILOX_M0) * (static_cast<uint32_t>(p1 >> 32) ^ tid ^ s.k0);
+  s.p_hi = static_cast<uint32_t>(p0 >> 32);
+  s.p_lo = static_cast<uint32_t>(p0);
+  s.x = static_cast<uint32_t>(p1) ^ (s.k0 + PHILOX_W0);
+  return s;
+}
+// Equals philox4x32<ROUNDS>(grp, tid, stream, 0, seed) (ROUNDS >= 2).
+template <int ROUNDS>
+__device__ __forceinline__ Philox4 philox4x32(const PhiloxStream& s, uint32_t grp) {
+  const uint64_t g = static_cast<uint64_t>(PHILOX_M0) * grp;                                     // round 1
+  const uint32_t n2 = static_cast<uint32_t>(g >> 32) ^ s.k1;
+  const uint64_t p = static_cast<uint64_t>(PHILOX_M1) * n2;                                      // round 2
+  uint32_t c0 = static_cast<uint32_t>(p >> 32) ^ s.x, c1 = static_cast<uint32_t>(p);
+  uint32_t c2 = s.p_hi ^ static_cast<uint32_t>(g) ^ (s.k1 + PHILOX_W1), c3 = s.p_lo;
+#pragma unroll
+  for (int r = 2; r < ROUNDS; ++r) {
+    const uint64_t p0 = static_cast<uint64_t>(PHILOX_M0) * c0;
+    const uint64_t p1 = static_cast<uint64_t>(PHILOX_M1) * c2;
+    const uint32_t n0 = static_cast<uint32_t>(p1 >> 32) ^ c1 ^ (s.k0 + r * PHILOX_W0);
+    c2 = static_cast<uint32_t>(p0 >> 32) ^ c3 ^ (s.k1 + r * PHILOX_W1);
+    c0 = n0; c1 = static_cast<uint32_t>(p1); c3 = static_cast<uint32_t>(p0);
+  }
+  return Philox4{c0, c1, c2, c3};
+}
+
 // Copy the 1024 pairs from global memory into the lane-replicated shared-memory layout
 // (entry i, lane l at byte i * 128 + l * 4).  All threads of the CTA call it; sync afterwards.
 __device__ __forceinline__ void gauss_table_to_smem(void* smem_tab, const uint32_t* gtab, int tid, int nthreads) {
@@ -107,19 +145,16 @@ __device__ __forceinline__ uint32_t gauss_pair(const char* base, uint32_t w) {
 
 // The 8 normals of a group as four bf16x2 registers (element 2j in the low half of word j).
 template <int SHIFT>
-__device__ __forceinline__ void gauss8_packed(const char* base, uint64_t seed, uint32_t tid, uint32_t grp,
-                                              uint32_t stream, uint32_t zp[4]) {
-  const Philox4 p = z_words(seed, tid, grp, stream);
+__device__ __forceinline__ void gauss8_packed(const char* base, const Philox4& p, uint32_t zp[4]) {
   zp[0] = gauss_pair<SHIFT>(base, p.x); zp[1] = gauss_pair<SHIFT>(base, p.y);
   zp[2] = gauss_pair<SHIFT>(base, p.z); zp[3] = gauss_pair<SHIFT>(base, p.w);
 }
 
 // The same 8 normals widened to fp32.
 template <int SHIFT>
-__device__ __forceinline__ void gauss8(const char* base, uint64_t seed, uint32_t tid, uint32_t grp,
-                                       uint32_t stream, float z[8]) {
+__device__ __forceinline__ void gauss8(const char* base, const Philox4& p, float z[8]) {
   uint32_t zp[4];
-  gauss8_packed<SHIFT>(base, seed, tid, grp, stream, zp);
+  gauss8_packed<SHIFT>(base, p, zp);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     z[2 * j] = __uint_as_float(zp[j] << 16);
@@ -135,10 +170,9 @@ __device__ __forceinline__ float gauss_scalar(const uint32_t* gtab, uint32_t u16
 // theta + c z for one 16-byte group of bf16 parameters: four fma.rn.bf16x2, each an exact
 // product and sum rounded once to bf16.  `c2` holds the coefficient (rounded to bf16) in both halves.
 template <int SHIFT>
-__device__ __forceinline__ uint4 perturb8_packed(const char* base, uint64_t seed, uint32_t tid,
-                                                 uint32_t grp, uint32_t c2, uint4 raw) {
+__device__ __forceinline__ uint4 perturb8_packed(const char* base, const Philox4& p, uint32_t c2, uint4 raw) {
   uint32_t zp[4];
-  gauss8_packed<SHIFT>(base, seed, tid, grp, 0u, zp);
+  gauss8_packed<SHIFT>(base, p, zp);
   uint32_t v[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -148,10 +182,10 @@ __device__ __forceinline__ uint4 perturb8_packed(const char* base, uint64_t seed
 
 // Both signs of the same perturbation from one draw of z: theta + c z and theta - c z (bf16x2, one rounding each).
 template <int SHIFT>
-__device__ __forceinline__ void perturb8_packed_dual(const char* base, uint64_t seed, uint32_t tid, uint32_t grp,
-                                                     uint32_t c2, uint4 raw, uint4& plus, uint4& minus) {
+__device__ __forceinline__ void perturb8_packed_dual(const char* base, const Philox4& p, uint32_t c2, uint4 raw,
+                                                     uint4& plus, uint4& minus) {
   uint32_t zp[4];
-  gauss8_packed<SHIFT>(base, seed, tid, grp, 0u, zp);
+  gauss8_packed<SHIFT>(base, p, zp);
   const uint32_t v[4] = {raw.x, raw.y, raw.z, raw.w};
   const uint32_t nc2 = c2 ^ 0x80008000u;          // -c in both halves
   uint32_t a[4], b[4];

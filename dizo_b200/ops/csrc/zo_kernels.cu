@@ -35,7 +35,6 @@ constexpr int ZO_CHUNK = 256;    // elements; tensor starts are aligned to this 
 constexpr int ZO_THREADS = 768;  // one persistent CTA (24 warps) per SM
 constexpr int ZO_THREADS_SMALL = 512;  // the variant that shares an SM with a GEMM CTA
 constexpr int ZO_SMEM_SMALL = GAUSS_BINS * 4;
-constexpr int ZO_UNROLL = 4;     // 16-byte loads in flight per lane
 constexpr int ZO_SMEM = GAUSS_SMEM_BYTES; // the lane-replicated inverse-CDF table
 
 struct ZoTensor {
@@ -90,22 +89,26 @@ __device__ __forceinline__ int find_tensor(const ZoTensor* tab, int lo, int hi, 
   return lo;
 }
 
-// One 256-element chunk: lane l owns elements [8l, 8l+8).  `raw` was loaded by the caller.
-template <bool Z2, bool BLEND, bool NORM, bool SR, int TS>
+// One 256-element chunk: lane l owns elements [8l, 8l+8).  `raw` was loaded by the caller.  zs, rs: the streams of z(seed1)
+// and of the rounding bits for this tensor; grp: this lane's Philox group.  FULL: the chunk lies inside the tensor (no
+// bounds to check, no padding to keep).
+template <bool Z2, bool BLEND, bool NORM, bool SR, bool DUAL, int TS, bool FULL>
 __device__ __forceinline__ void zo_chunk(const ZoSweepArgs& a, const ZoTensor& t, float alpha,
-                                         long long cpos, int lane, const uint4 raw,
+                                         long long cpos, int lane, const uint4 raw, const PhiloxStream& zs,
+                                         const PhiloxStream& rs, const uint32_t grp,
                                          const char* tab, float c1, float c2, uint32_t c1_pair) {
   const long long e0 = cpos - t.offset + lane * 8;  // element inside this piece
   float sq = 0.f;
   constexpr bool PACKED = !Z2 && !BLEND && !NORM && !SR;
   if (PACKED) {
-    if (e0 < t.numel) {
+    if (FULL || e0 < t.numel) {
       uint4 o = raw, o2 = raw;
       if (c1 != 0.f) {
-        if (a.dst2) perturb8_packed_dual<TS>(tab, a.seed1, t.tensor_id, zo_group(t, e0), c1_pair, raw, o, o2);
-        else o = perturb8_packed<TS>(tab, a.seed1, t.tensor_id, zo_group(t, e0), c1_pair, raw);
+        const Philox4 zw = philox4x32<Z_PHILOX_ROUNDS>(zs, grp);
+        if (DUAL) perturb8_packed_dual<TS>(tab, zw, c1_pair, raw, o, o2);
+        else o = perturb8_packed<TS>(tab, zw, c1_pair, raw);
       }
-      if (e0 + 8 > t.numel) {
+      if (!FULL && e0 + 8 > t.numel) {
         // ragged tail of a tensor: keep the padding elements as they were
         uint32_t ov[4] = {o.x, o.y, o.z, o.w};
         uint32_t ov2[4] = {o2.x, o2.y, o2.z, o2.w};
@@ -123,14 +126,14 @@ __device__ __forceinline__ void zo_chunk(const ZoSweepArgs& a, const ZoTensor& t
       }
       uint4* dp = reinterpret_cast<uint4*>(a.dst + (cpos + lane * 8 - a.dst_shift));
       if (DZ_STORE_OK(dp, 16)) *dp = o;
-      if (a.dst2) {
+      if (DUAL) {
         uint4* dp2 = reinterpret_cast<uint4*>(a.dst2 + (cpos + lane * 8 - a.dst_shift));
         if (DZ_STORE_OK(dp2, 16)) *dp2 = o2;
       }
     }
     return;
   }
-  if (e0 < t.numel) {
+  if (FULL || e0 < t.numel) {
     const long long pos = cpos + lane * 8;
     float v[8] = {bf16_lo(raw.x), bf16_hi(raw.x), bf16_lo(raw.y), bf16_hi(raw.y),
                   bf16_lo(raw.z), bf16_hi(raw.z), bf16_lo(raw.w), bf16_hi(raw.w)};
@@ -145,36 +148,34 @@ __device__ __forceinline__ void zo_chunk(const ZoSweepArgs& a, const ZoTensor& t
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = fmaf(alpha, v[j] - an[j], an[j]);
     }
-    const uint32_t grp = zo_group(t, e0);
     if (c1 != 0.f) {
       float z[8];
-      gauss8<TS>(tab, a.seed1, t.tensor_id, grp, 0u, z);
+      gauss8<TS>(tab, philox4x32<Z_PHILOX_ROUNDS>(zs, grp), z);
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = fmaf(c1, z[j], v[j]);
     }
     if (Z2) {
       float z[8];
-      gauss8<TS>(tab, a.seed2, t.tensor_id, grp, 0u, z);
+      gauss8<TS>(tab, z_words(a.seed2, t.tensor_id, grp, 0u), z);
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] = fmaf(c2, z[j], v[j]);
     }
     uint32_t o[4];
     if (SR) {
       // stochastic rounding: add 16 random bits below the bf16 mantissa, truncate
-      Philox4 rb = philox4x32<Z_PHILOX_ROUNDS>(grp, t.tensor_id, 1u, 0u, static_cast<uint32_t>(a.sr_seed),
-                                  static_cast<uint32_t>(a.sr_seed >> 32));
+      const Philox4 rb = philox4x32<Z_PHILOX_ROUNDS>(rs, grp);
       uint32_t rw[4] = {rb.x, rb.y, rb.z, rb.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         uint32_t lo = __float_as_uint(v[2 * j]) + (rw[j] & 0xffffu);
         uint32_t hi = __float_as_uint(v[2 * j + 1]) + (rw[j] >> 16);
-        o[j] = (lo >> 16) | (hi & 0xffff0000u);
+        o[j] = __byte_perm(lo, hi, 0x7632);
       }
     } else {
 #pragma unroll
       for (int j = 0; j < 4; ++j) o[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
     }
-    if (e0 + 8 > t.numel) {
+    if (!FULL && e0 + 8 > t.numel) {
       // ragged tail of a tensor: keep the padding elements as they were
       const uint32_t rawv[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
@@ -191,7 +192,7 @@ __device__ __forceinline__ void zo_chunk(const ZoSweepArgs& a, const ZoTensor& t
       // norm of what was stored (the bf16 values), so it equals a later re-read
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        if (e0 + j < t.numel) {
+        if (FULL || e0 + j < t.numel) {
           float w = (j & 1) ? bf16_hi(o[j >> 1]) : bf16_lo(o[j >> 1]);
           float d = w - an[j];
           sq = fmaf(d, d, sq);
@@ -211,19 +212,24 @@ __device__ __forceinline__ void zo_chunk(const ZoSweepArgs& a, const ZoTensor& t
 }
 
 // Persistent: one CTA of 24 warps per SM.  The inverse-CDF table sits in shared memory (replicated per
-// lane, conflict-free); every warp owns a contiguous run of chunks and works on ZO_UNROLL chunks at a
-// time while the loads of the next ZO_UNROLL chunks are already in flight (register double buffering:
+// lane, conflict-free); every warp owns a contiguous run of chunks and works on UNROLL chunks at a
+// time while the loads of the next UNROLL chunks are already in flight (register double buffering:
 // 2 x 64 bytes per lane, ~100 KB per SM), so HBM latency is covered while z is computed.
+// Chunks inside a tensor run without bounds checks, with the tensor's share of the first two Philox rounds
+// computed once; 512 Mi parameters, before and now: one perturbed copy 0.509 / 0.386 ms (6.1 TB/s), both signs 0.596 /
+// 0.588 (6.0; two chunks at a time - four measured 0.624, the two store streams then run further apart), the
+// stochastically rounded update 0.704 / 0.592 (4.0: two Philox calls per 16 bytes bound it).
 //
 // SMALL: the variant that runs beside a GEMM.  Its table is the plain 4 KB copy (bank conflicts
 // instead of 128 KB of shared memory) and it is bounded to 512 threads x 64 registers, so one of its
 // CTAs fits on an SM that already holds a GEMM CTA (~200 KB of shared memory, 192 threads): launched on
 // a second stream it sweeps the next layer in the shadow of the tensor-core work, which leaves the
 // issue slots and HBM almost idle.
-template <bool Z2, bool BLEND, bool NORM, bool SR, bool SMALL>
+template <bool Z2, bool BLEND, bool NORM, bool SR, bool SMALL, bool DUAL>
 __global__ void __launch_bounds__(SMALL ? ZO_THREADS_SMALL : ZO_THREADS, SMALL ? 2 : 1)
 zo_sweep_kernel(const ZoSweepArgs a_in) {
   constexpr int THREADS = SMALL ? ZO_THREADS_SMALL : ZO_THREADS;
+  constexpr int UNROLL = DUAL ? 2 : 4;              // 16-byte loads in flight per lane
   constexpr int TS = SMALL ? 2 : 7;                 // log2 bytes between table entries
   ZoSweepArgs a = a_in;
   if (a.seed1_dev) {
@@ -260,9 +266,11 @@ zo_sweep_kernel(const ZoSweepArgs a_in) {
   long long t_next = (cur + 1 < a.t_end) ? a.table[cur + 1].offset : (1ll << 62);
   float alpha = 1.f;
   if (BLEND && t.slot >= 0) alpha = __ldg(a.alpha + t.slot);
+  PhiloxStream zs = philox_stream(a.seed1, t.tensor_id, 0u), rs = zs;
+  if (SR) rs = philox_stream(a.sr_seed, t.tensor_id, 1u);
 
-  uint4 nxt[ZO_UNROLL];
-  bool have = false;           // nxt holds the chunks [chunk, chunk + ZO_UNROLL)
+  uint4 nxt[UNROLL];
+  bool have = false;           // nxt holds the chunks [chunk, chunk + UNROLL)
   while (chunk < chunk_stop) {
     const long long cpos = chunk * ZO_CHUNK;
     if (cpos >= t_next) {
@@ -271,36 +279,130 @@ zo_sweep_kernel(const ZoSweepArgs a_in) {
       t = a.table[cur];
       t_next = (cur + 1 < a.t_end) ? a.table[cur + 1].offset : (1ll << 62);
       if (BLEND && t.slot >= 0) alpha = __ldg(a.alpha + t.slot);
+      zs = philox_stream(a.seed1, t.tensor_id, 0u);
+      if (SR) rs = philox_stream(a.sr_seed, t.tensor_id, 1u);
     }
-    // ZO_UNROLL full chunks of this tensor, inside this warp's run, start at chunk c
+    // UNROLL full chunks of this tensor, inside this warp's run, start at chunk c
     const long long full_end = t.offset + (t.numel / ZO_CHUNK) * ZO_CHUNK;
-    const bool fast = chunk + ZO_UNROLL <= chunk_stop && cpos + ZO_UNROLL * ZO_CHUNK <= full_end;
+    const bool fast = chunk + UNROLL <= chunk_stop && cpos + UNROLL * ZO_CHUNK <= full_end;
     if (fast) {
-      uint4 raw[ZO_UNROLL];
+      uint4 raw[UNROLL];
 #pragma unroll
-      for (int u = 0; u < ZO_UNROLL; ++u)
+      for (int u = 0; u < UNROLL; ++u)
         raw[u] = have ? nxt[u] : *reinterpret_cast<const uint4*>(a.src + cpos + u * ZO_CHUNK + lane * 8);
-      const long long npos = cpos + ZO_UNROLL * ZO_CHUNK;
+      const long long npos = cpos + UNROLL * ZO_CHUNK;
       // (the small variant has time to spare and registers to save: it does not prefetch)
-      have = !SMALL && chunk + 2 * ZO_UNROLL <= chunk_stop && npos + ZO_UNROLL * ZO_CHUNK <= full_end;
+      have = !SMALL && chunk + 2 * UNROLL <= chunk_stop && npos + UNROLL * ZO_CHUNK <= full_end;
       if (have) {
 #pragma unroll
-        for (int u = 0; u < ZO_UNROLL; ++u)
+        for (int u = 0; u < UNROLL; ++u)
           nxt[u] = *reinterpret_cast<const uint4*>(a.src + npos + u * ZO_CHUNK + lane * 8);
       }
+      // a contiguous piece advances by 32 groups per chunk (elem_base is a multiple of 8)
+      const uint32_t grp0 = static_cast<uint32_t>((t.elem_base + (cpos - t.offset)) >> 3) + lane;
 #pragma unroll
-      for (int u = 0; u < ZO_UNROLL; ++u)
-        zo_chunk<Z2, BLEND, NORM, SR, TS>(a, t, alpha, cpos + u * ZO_CHUNK, lane, raw[u], tab, c1, c2, c1_pair);
-      chunk += ZO_UNROLL;
+      for (int u = 0; u < UNROLL; ++u) {
+        const uint32_t grp = t.local_cols ? zo_group(t, cpos + u * ZO_CHUNK - t.offset + lane * 8) : grp0 + u * 32;
+        zo_chunk<Z2, BLEND, NORM, SR, DUAL, TS, true>(a, t, alpha, cpos + u * ZO_CHUNK, lane, raw[u], zs, rs, grp, tab, c1, c2,
+                                                c1_pair);
+      }
+      chunk += UNROLL;
     } else {
       uint4 raw = make_uint4(0, 0, 0, 0);
       if (cpos - t.offset + lane * 8 < t.numel)
         raw = *reinterpret_cast<const uint4*>(a.src + cpos + lane * 8);
-      zo_chunk<Z2, BLEND, NORM, SR, TS>(a, t, alpha, cpos, lane, raw, tab, c1, c2, c1_pair);
+      zo_chunk<Z2, BLEND, NORM, SR, DUAL, TS, false>(a, t, alpha, cpos, lane, raw, zs, rs,
+                                               zo_group(t, cpos - t.offset + lane * 8), tab, c1, c2, c1_pair);
       chunk += 1;
       have = false;
     }
   }
+}
+
+// Blend without perturbation (the gamma-search forwards and the projection): dst = anchor + alpha[slot] (theta - anchor)
+// for slotted tensors, a copy of the others.  No z, so no 128 KB table and no 24-warp CTA: a plain streaming kernel,
+// ZB_UNROLL chunks of theta and theta_0 in flight per warp.  512 Mi parameters: 0.766 -> 0.612 ms (5.8 TB/s).
+constexpr int ZB_THREADS = 256;
+constexpr int ZB_UNROLL = 4;
+struct ZoBlendArgs {
+  const __nv_bfloat16* src;
+  __nv_bfloat16* dst;
+  long long dst_shift;
+  const __nv_bfloat16* anchor;
+  const ZoTensor* table;
+  int t_begin, t_end;
+  long long chunk_begin, chunk_end;
+  const float* alpha;
+};
+
+__device__ __forceinline__ uint4 blend8(const uint4& t, const uint4& n, float alpha) {
+  const uint32_t tv[4] = {t.x, t.y, t.z, t.w}, nv[4] = {n.x, n.y, n.z, n.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    o[j] = pack_bf16x2(fmaf(alpha, bf16_lo(tv[j]) - bf16_lo(nv[j]), bf16_lo(nv[j])),
+                       fmaf(alpha, bf16_hi(tv[j]) - bf16_hi(nv[j]), bf16_hi(nv[j])));
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// The first `keep` elements of `a`, the rest (padding behind a tensor) of `raw`.
+__device__ __forceinline__ uint4 keep_tail(const uint4& a, const uint4& raw, int keep) {
+  const uint32_t av[4] = {a.x, a.y, a.z, a.w}, rv[4] = {raw.x, raw.y, raw.z, raw.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint32_t m = keep >= 2 * j + 2 ? 0xffffffffu : keep == 2 * j + 1 ? 0xffffu : 0u;
+    o[j] = (av[j] & m) | (rv[j] & ~m);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+__global__ void __launch_bounds__(ZB_THREADS)
+zo_blend_kernel(const ZoBlendArgs a) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = (long long)gridDim.x * (ZB_THREADS / 32);
+  const long long w0 = a.chunk_begin + (long long)blockIdx.x * (ZB_THREADS / 32) + (threadIdx.x >> 5);
+  for (long long c0 = w0; c0 < a.chunk_end; c0 += warps * ZB_UNROLL) {
+    uint4 raw[ZB_UNROLL], anc[ZB_UNROLL];
+    int slot[ZB_UNROLL], keep[ZB_UNROLL];
+#pragma unroll
+    for (int u = 0; u < ZB_UNROLL; ++u) {
+      const long long chunk = c0 + u * warps;
+      slot[u] = -1;
+      keep[u] = 0;
+      if (chunk < a.chunk_end) {
+        const ZoTensor& t = a.table[find_tensor(a.table, a.t_begin, a.t_end, chunk * ZO_CHUNK)];
+        const long long e0 = chunk * ZO_CHUNK - t.offset + lane * 8;
+        const long long left = t.numel - e0;
+        keep[u] = left <= 0 ? 0 : left >= 8 ? 8 : (int)left;
+        if (keep[u]) {
+          slot[u] = t.slot;
+          raw[u] = *reinterpret_cast<const uint4*>(a.src + chunk * ZO_CHUNK + lane * 8);
+          if (t.slot >= 0) anc[u] = *reinterpret_cast<const uint4*>(a.anchor + t.anchor_offset + e0);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < ZB_UNROLL; ++u) {
+      if (!keep[u]) continue;
+      const long long at = (c0 + u * warps) * ZO_CHUNK + lane * 8 - a.dst_shift;
+      uint4 o = raw[u];
+      if (slot[u] >= 0) o = keep_tail(blend8(raw[u], anc[u], __ldg(a.alpha + slot[u])), raw[u], keep[u]);
+      uint4* dp = reinterpret_cast<uint4*>(a.dst + at);
+      if (DZ_STORE_OK(dp, 16)) *dp = o;
+    }
+  }
+}
+
+static int launch_blend(const ZoBlendArgs& a, cudaStream_t stream) {
+  const long long chunks = a.chunk_end - a.chunk_begin;
+  if (chunks <= 0) return DZ_OK;
+  const long long per_cta = (ZB_THREADS / 32) * ZB_UNROLL;
+  long long blocks = (chunks + per_cta - 1) / per_cta;
+  const long long cap = 8LL * sm_count();
+  if (blocks > cap) blocks = cap;
+  zo_blend_kernel<<<(unsigned)blocks, ZB_THREADS, 0, stream>>>(a);
+  return cuda_rc(cudaGetLastError());
 }
 
 // Sum the per-chunk partials of each slotted tensor in fixed order: sq[slot] = sum.
@@ -373,11 +475,11 @@ __global__ void scalar_diff_kernel(const float* a, const float* b, float scale, 
   out[0] = (a[0] - b[0]) * scale;
 }
 
-template <bool Z2, bool BLEND, bool NORM, bool SR, bool SMALL = false>
+template <bool Z2, bool BLEND, bool NORM, bool SR, bool SMALL = false, bool DUAL = false>
 static int launch_sweep(const ZoSweepArgs& a, cudaStream_t stream) {
   long long chunks = a.chunk_end - a.chunk_begin;
   if (chunks <= 0) return DZ_OK;
-  auto kern = zo_sweep_kernel<Z2, BLEND, NORM, SR, SMALL>;
+  auto kern = zo_sweep_kernel<Z2, BLEND, NORM, SR, SMALL, DUAL>;
   constexpr int threads = SMALL ? ZO_THREADS_SMALL : ZO_THREADS;
   constexpr int smem = SMALL ? ZO_SMEM_SMALL : ZO_SMEM;
   if (!SMALL) {
@@ -426,6 +528,12 @@ extern "C" int dz_zo_sweep_seeded(const void* src, void* dst, long long dst_shif
   a.alpha = alpha; a.chunk_sq = chunk_sq; a.sr_seed = sr_seed;
   a.gauss_table = (const uint32_t*)gauss_table;
   int key = (z2 ? 1 : 0) | (blend ? 2 : 0) | (norm ? 4 : 0) | (sr ? 8 : 0);
+  if (key == 2 && !small && c1 == 0.f) {
+    ZoBlendArgs b{};
+    b.src = a.src; b.dst = a.dst; b.dst_shift = dst_shift; b.anchor = a.anchor; b.table = a.table;
+    b.t_begin = t_begin; b.t_end = t_end; b.chunk_begin = chunk_begin; b.chunk_end = chunk_end; b.alpha = alpha;
+    return launch_blend(b, stream);
+  }
   if (small) {
     if (key == 0) return launch_sweep<false, false, false, false, true>(a, stream);
     if (key == 2) return launch_sweep<false, true, false, false, true>(a, stream);
@@ -474,8 +582,8 @@ extern "C" int dz_zo_sweep_dual(const void* src, void* dst_plus, void* dst_minus
   a.t_begin = t_begin; a.t_end = t_end; a.chunk_begin = chunk_begin; a.chunk_end = chunk_end;
   a.seed1 = seed1; a.seed1_dev = seed1_dev; a.c1 = c1; a.c1_ptr = c1_ptr;
   a.gauss_table = (const uint32_t*)gauss_table;
-  if (small) return launch_sweep<false, false, false, false, true>(a, stream);
-  return launch_sweep<false, false, false, false>(a, stream);
+  if (small) return launch_sweep<false, false, false, false, true, true>(a, stream);
+  return launch_sweep<false, false, false, false, false, true>(a, stream);
 }
 
 extern "C" int dz_zo_reduce_chunks(const void* table, int num_tensors, const float* chunk_sq,
@@ -511,7 +619,7 @@ __global__ void zo_fill_z_kernel(float* out, long long numel, long long elem_bas
   long long e0 = g * 8;
   if (e0 >= numel) return;
   float z[8];
-  gauss8<2>(reinterpret_cast<const char*>(tab), seed, tensor_id, (uint32_t)((elem_base + e0) >> 3), 0u, z);
+  gauss8<2>(reinterpret_cast<const char*>(tab), z_words(seed, tensor_id, (uint32_t)((elem_base + e0) >> 3), 0u), z);
   for (int j = 0; j < 8 && e0 + j < numel; ++j)
     if (DZ_STORE_OK(out + e0 + j, 4)) out[e0 + j] = z[j];
 }

@@ -405,3 +405,39 @@ def test_sampling_kernel_distribution_and_filters():
     # different steps draw differently, same (seed, offset) repeats
     a, b, c = sample(big, seed=9, offset=0), sample(big, seed=9, offset=0), sample(big, seed=9, offset=1)
     assert torch.equal(a, b) and not torch.equal(a, c)
+
+
+@pytest.mark.parametrize("sizes", [(1,), (255, 256, 257), (8, 1027, 40960, 5), (262144 + 3, 7, 65536)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_blend_sweep_over_ragged_pieces(sizes, in_place):
+    """theta_0 + alpha (theta - theta_0) of the slotted pieces, the others and the padding behind every piece as they were."""
+    from dizo_b200.ops.zo import ParamArena, Piece
+    ar = ParamArena([Piece(f"p{i}", (n,), i) for i, n in enumerate(sizes)], "cuda", torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(sum(sizes))
+    ar.data.copy_(torch.randn(ar.data.shape, device="cuda", generator=g))
+    ar.set_dizo([f"p{i}" for i in range(0, len(sizes), 2)])
+    theta0 = ar.data.double()
+    ar.data.add_((torch.randn(ar.data.shape, device="cuda", generator=g) * 0.1).bfloat16())
+    before = ar.data.clone()
+    alpha = torch.rand(ar.n_slots, device="cuda", generator=g) * 2
+    dst = None if in_place else torch.full_like(ar.data, 7.0)
+    ar.sweep(alpha=alpha, dst=dst)
+    got = ar.data if in_place else dst
+    assert in_place or torch.equal(ar.data, before)
+    inside = torch.zeros(ar.data.numel(), dtype=torch.bool, device="cuda")
+    for p in ar.pieces:
+        r = slice(p.offset, p.offset + p.numel)
+        inside[r] = True
+        if p.slot < 0:
+            assert torch.equal(got[r], before[r])
+            continue
+        want = theta0[r] + alpha[p.slot].double() * (before[r].double() - theta0[r])
+        # one fp32 difference and one fp32 fma (2^-24 each, of the terms), then one rounding to bf16 (2^-8 of the result)
+        terms = theta0[r].abs() + alpha[p.slot].double() * (before[r].double() - theta0[r]).abs()
+        assert ((got[r].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -22 * terms).all()
+    # a group of 8 that starts inside a piece may be stored whole (with the padding it had); nothing else is touched
+    if in_place:
+        assert torch.equal(got[~inside], before[~inside])
+    else:
+        out = ~inside & (got != 7.0)
+        assert torch.equal(got[out], before[out])
