@@ -28,6 +28,7 @@ from typing import Callable, Iterable
 import torch
 
 from ..ops import attention as attn_ops
+from ..ops import block as block_ops
 from ..ops import gemm, loss as loss_ops, norm, peft as peft_ops
 from ..ops.zo import ParamArena, Piece
 
@@ -280,6 +281,7 @@ class OPTModel:
         self._where = {p.name: self.arena for p in self.arena.pieces}
         self._where.update({p.name: self.frozen for p in self.frozen.pieces})
         self._staging: dict = {}
+        self._block_plans: dict = {}
         self._side = None
         self._merge_buf: dict = {}
         # LoRA: k_proj.weight is frozen, so its copy inside a layer's merged QKV operand stays valid
@@ -618,6 +620,51 @@ class OPTModel:
             h = norm.layernorm(h, w.ln2_w, w.ln2_b, cfg.layer_norm_eps)
         return h
 
+    # ------------------------------------------------------------------ blocks as native calls
+    def _block_runner(self, batch: Batch) -> "block_ops.BlockRunner | None":
+        """Runs whole blocks of this forward natively; None where :meth:`_layer_forward` has to (CPU, adapters, another
+        architecture or layout, forwards that record the QKV activations)."""
+        cfg = self.config
+        if (self.device.type != "cuda" or self.dtype != torch.bfloat16 or self.use_lora or self.use_prefix
+                or self.kv_capture is not None or gemm._VARIANT != 0
+                or type(self)._layer_forward is not OPTModel._layer_forward
+                or type(self)._layer_weights is not OPTModel._layer_weights
+                or type(self).hidden_states is not OPTModel.hidden_states):
+            return None
+        B, L = batch.input_ids.shape
+        return block_ops.BlockRunner(B, L, cfg.hidden_size, cfg.ffn_dim, cfg.num_attention_heads,
+                                     cfg.do_layer_norm_before, gemm.ACT[cfg.activation_function], cfg.layer_norm_eps,
+                                     batch.pad_left, self.device)
+
+    def _block_weights(self, i: int, staged: torch.Tensor | None, shift: int, whole: bool) -> list[int] | None:
+        """Addresses of block ``i``'s weights in the order of ``ops.block.WEIGHTS``: in ``staged`` (a buffer laid out like
+        the arena from element ``shift`` on) the whole block, or with ``whole`` False its q | k | v weights only.  None
+        where q, k and v are not adjacent.  Only offsets are kept between calls."""
+        plan = self._block_plans.get(i)
+        if plan is None:
+            lp = layer_prefix(i)
+            names = ["self_attn_layer_norm.weight", "self_attn_layer_norm.bias", "self_attn.q_proj.weight",
+                     "self_attn.q_proj.bias", "self_attn.out_proj.weight", "self_attn.out_proj.bias",
+                     "final_layer_norm.weight", "final_layer_norm.bias", "fc1.weight", "fc1.bias", "fc2.weight", "fc2.bias"]
+            plan = []
+            for n in names:
+                ar = self._where[lp + n]
+                plan.append((ar, ar.pieces[ar.index[lp + n]].offset, n.endswith("q_proj.weight")))
+            for wb in ("weight", "bias"):
+                ps = [self._where[f"{lp}self_attn.{x}_proj.{wb}"] for x in "qkv"]
+                pc = [ar.pieces[ar.index[f"{lp}self_attn.{x}_proj.{wb}"]] for ar, x in zip(ps, "qkv")]
+                if any(ar is not ps[0] for ar in ps) or any(b.offset != a.offset + a.numel for a, b in zip(pc, pc[1:])):
+                    plan = False
+                    break
+            self._block_plans[i] = plan
+        if plan is False:
+            return None
+        base = {id(ar): ar.data.data_ptr() for ar in (self.arena, self.frozen)}
+        if staged is None:
+            return [base[id(ar)] + 2 * off for ar, off, _ in plan]
+        s0 = staged.data_ptr() - 2 * shift
+        return [s0 + 2 * off if ar is self.arena and (whole or qkv) else base[id(ar)] + 2 * off for ar, off, qkv in plan]
+
     @torch.no_grad()
     def hidden_states(self, batch: Batch, transform: Transform | None = None,
                       rows: torch.Tensor | None = None) -> torch.Tensor:
@@ -660,6 +707,8 @@ class OPTModel:
                 shift = self._sweep_group(i, transform, buf)
             return buf, shift
 
+        runner = None if overlap else self._block_runner(batch)
+        owned = False                       # h is a buffer of this forward: a block may write its output over it
         pending = None
         if use_t and nl > 0 and has_group.get(0):
             if overlap:
@@ -676,8 +725,15 @@ class OPTModel:
             # queue the next layer's sweep first: it runs beside this layer's GEMMs
             if use_t and i + 1 < nl and has_group.get(i + 1):
                 pending = launch_transform(i + 1)
-            w = self._layer_weights(i, self._resolver(i, transform, staged, shift))
             only = rows if (i == nl - 1 and self.kv_capture is None) else None
+            if runner is not None and only is None:
+                whole = staged is None or self._blend_range(i, transform) is None
+                ptrs = self._block_weights(i, staged, shift, whole)
+                if ptrs is not None:
+                    h = runner.run(h, ptrs, out=h if owned else None)
+                    owned = True
+                    continue
+            w = self._layer_weights(i, self._resolver(i, transform, staged, shift))
             h = self._layer_forward(h, w, batch, only)
             if overlap and has_group.get(i):
                 ev = torch.cuda.Event()
@@ -805,16 +861,28 @@ class OPTModel:
         h0 = self._embed(batch.input_ids, batch.positions, ggets[0])
         hs = [h0, h0 if same else self._embed(batch.input_ids, batch.positions, ggets[1])]
         layer_numel = max((self.arena.group_numel(g) for g in groups if g >= 0), default=0)
+        runner = self._block_runner(batch)
+        owned = [False, False]              # hs[s] is a buffer of this forward that no other stream reads
         for i in range(nl):
             only = batch.rows if i == nl - 1 else None
+            staged, shift = (None, None), 0
             if i in groups:
-                same = False
+                if same:
+                    same, owned = False, [False, False]        # both streams read the one buffer so far
                 b1 = self._staging_for(("layer", i % 2), layer_numel)
                 b2 = self._staging_for(("layer-", i % 2), layer_numel)
                 shift = self._sweep_group(i, tr, b1, dst2=b2)
-                gets = [self._resolver(i, tr, b1, shift), self._resolver(i, tr, b2, shift)]
-            else:
-                gets = [self._resolver(i, None, None, 0)] * 2
+                staged = (b1, b2)
+            if runner is not None and only is None:
+                ptrs = [self._block_weights(i, b, shift, True) for b in staged]
+                if ptrs[0] is not None:
+                    for s in range(1 if same else 2):
+                        hs[s] = runner.run(hs[s], ptrs[s], out=hs[s] if owned[s] else None)
+                        owned[s] = True
+                    if same:
+                        hs[1] = hs[0]
+                    continue
+            gets = [self._resolver(i, None if b is None else tr, b, shift) for b in staged]
             if same:
                 h0 = self._layer_forward(hs[0], self._layer_weights(i, gets[0]), batch, only)
                 hs = [h0, h0]

@@ -105,16 +105,6 @@ def linear_qkv_rope(x: torch.Tensor, w_qkv: torch.Tensor, L: int, pos0: int, H: 
     return out
 
 
-def _skinny_pays(M: int, N: int) -> bool:
-    """Whether the swapped-operand, K-split kernel takes a product with M rows and N columns.  Up to 16 rows it always
-    wins (one row, us, 128-row tiles / skinny: N 2048 K 8192 32.9 / 10.5, N 50272 K 2048 59.1 / 36.3).  With more rows its
-    wider activation operand costs L2 traffic per tile of W, which only K splitting makes up for: at 32 rows N 32000 K
-    4096 50.2 / 48.1 but N 50272 K 2048 40.6 / 42.8; at 64 rows N 2048 K 8192 31.9 / 13.7, N 8192 K 2048 12.4 / 11.9, but
-    N 16384 K 4096 29.2 / 29.6 and N 50272 K 2048 40.4 / 49.5."""
-    tiles = (N + 127) // 128
-    return 0 < M <= 16 or (M <= 32 and tiles <= 296) or (M <= SKINNY_ROWS and tiles <= 74)
-
-
 def _skinny(x2, w, out2, bias, res2, act: int, scale: float, splits: int = 0) -> None:
     """``out2 = epilogue(x2 @ w.T)`` for at most ``SKINNY_ROWS`` rows (``act`` 3: SwiGLU over gate | up rows of w)."""
     rc = _lib.lib().dz_gemm_skinny(
@@ -132,7 +122,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, a
            tile_n: int = 0) -> torch.Tensor:
     """x [..., K] (bf16), w [N, K] (bf16) -> [..., N] in ``out_dtype`` (bf16 or fp32).
 
-    ``tile_n``: 0 = choose, 128 / 256 = one-SM kernel with that tile width, 512 = two-SM kernel."""
+    ``tile_n``: 0 = choose (``dz_linear`` in ``csrc/block_forward.cu``), 128 / 256 = one-SM kernel with that tile width, 512 = two-SM kernel."""
     if not x.is_cuda:
         y = linear_reference(x, w, bias, act, residual, scale, out_dtype)
         if out is not None:
@@ -160,16 +150,19 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, a
     if M == 0:
         return out.reshape(*x.shape[:-1], N)
     variant = _VARIANT
-    if variant == 0 and tile_n == 0 and _skinny_pays(M, N):
-        _skinny(x2, w, out2, bias, res2, ACT[act], scale)
-        return out.reshape(*x.shape[:-1], N)
     if tile_n == 512:
         variant, tile_n = 2, 0
     elif tile_n in (128, 256):
         variant = 1
     if variant == 0:
-        # pairs of SMs (256 x 256 tiles) once there is work for most of them
-        variant = 2 if (M >= 256 and ((M + 255) // 256) * ((N + 255) // 256) >= 48) else 1
+        rc = _lib.lib().dz_linear(
+            _lib.ptr(x2), ctypes.c_longlong(x2.stride(0)), _lib.ptr(w), ctypes.c_longlong(w.stride(0)),
+            _lib.ptr(out2), ctypes.c_longlong(out2.stride(0)), _lib.ptr(bias), _lib.ptr(res2),
+            ctypes.c_longlong(res2.stride(0) if res2 is not None else 0),
+            M, N, K, ACT[act], int(out_dtype == torch.float32), ctypes.c_float(scale),
+            _lib.ptr(_lib.err_word(x.device)), _lib.stream_ptr())
+        _lib.check(rc, "dz_linear")
+        return out.reshape(*x.shape[:-1], N)
     if variant == 2:
         rc = _lib.lib().dz_gemm2_bf16_tn(
             _lib.ptr(x2), ctypes.c_longlong(x2.stride(0)), _lib.ptr(w), ctypes.c_longlong(w.stride(0)),
