@@ -37,12 +37,28 @@ static bool skinny_pays(int M, int N) {
   return M <= 16 || (M <= 32 && tiles <= 296) || (M <= 64 && tiles <= 74);
 }
 
+// CTAs per 128 x 128 tile where the K-split kernel pays for more rows than that, else 0: few tiles, and enough K blocks
+// that the halved loop is worth the reduction over the cluster.  Launches beyond about 128 CTAs of split tiles, or clusters
+// of 8, do not pack and run in two rounds.  Measured, us, 128-row tiles / split (CTAs a tile): M 360 N 1024 K 4096 17.9 /
+// 11.6 (4), M 512 N 1024 K 4096 17.7 / 12.1 (4), M 128 N 2048 K 8192 32.3 / 13.8 (6), M 100 N 4096 K 16384 62.1 / 32.4 (4),
+// M 300 N 2048 K 8192 31.5 / 23.9 (2), M 1000 N 1024 K 4096 17.8 / 16.7 (2); but M 360 N 1024 K 1024 7.2 / 8.4 (4), M 1024
+// N 768 K 768 7.4 / 10.3 (3), M 300 N 2048 K 2048 11.5 / 13.1 (2).
+static int split_pays(int M, int N, int K) {
+  const long long tiles = (long long)((M + 127) / 128) * ((N + 127) / 128);
+  const int num_kb = (K + 63) / 64;
+  if (tiles <= 32 && num_kb >= 32) return tiles <= 21 ? 6 : 4;
+  return tiles <= 64 && num_kb >= 64 ? 2 : 0;
+}
+
 extern "C" int dz_linear(const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo,
                          const void* bias, const void* residual, long long ldr, int M, int N, int K, int act,
                          int out_fp32, float out_scale, uint32_t* err, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return DZ_ERR_ARG;
-  if (skinny_pays(M, N))
-    return dz_gemm_skinny(A, lda, W, ldw, out, ldo, bias, residual, ldr, M, N, K, act, out_fp32, out_scale, 0, err, stream);
+  const bool skinny = skinny_pays(M, N);
+  const int splits = skinny || M <= 64 ? 0 : split_pays(M, N, K);
+  if (skinny || splits)
+    return dz_gemm_skinny(A, lda, W, ldw, out, ldo, bias, residual, ldr, M, N, K, act, out_fp32, out_scale, splits, err,
+                          stream);
   // pairs of SMs (256-row tiles) once there is work for most of them
   if (M >= 256 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= 48)
     return dz_gemm2_bf16_tn(A, lda, W, ldw, out, ldo, bias, residual, ldr, M, N, K, act, out_fp32, out_scale, err, stream);

@@ -8,11 +8,11 @@
 
 namespace dz {
 
-constexpr int SK_MAX_ROWS = 64;      // activation rows a launch takes
+constexpr int SK_MAX_ROWS = 64;      // sequences of a decoding step
 
 struct SkinnyArgs {
   int M, N, K;                       // N: columns written (half the rows of W for act 3)
-  int splits, kb_per_cta, num_kb;
+  int splits, kb_per_cta, num_kb, num_n;
   void* out;                         // bf16 or fp32 [M, ldo]
   long long ldo;
   const __nv_bfloat16* bias;         // [N] or null

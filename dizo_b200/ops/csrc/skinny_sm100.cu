@@ -1,4 +1,4 @@
-// GEMM for a handful of activation rows on sm_100a:  out[M,N] = epilogue( A[M,K] * W[N,K]^T ),  M <= 64.
+// GEMM for few output tiles on sm_100a:  out[M,N] = epilogue( A[M,K] * W[N,K]^T ), K split over a cluster of CTAs.
 //
 // Decoding, the option rows of a loss and the last block's tail multiply a few rows with whole weight matrices: the
 // bytes of W bound the time and the only question is how to keep enough of them in flight on every SM.  The 128-row
@@ -11,6 +11,9 @@
 //     through distributed shared memory in a fixed order (deterministic, no workspace, no second launch);
 //   * two CTAs fit on an SM (about 108 KB each), so the next launch of a decoding step can fill its ring while this one
 //     drains (programmatic dependent launch; `w_static` says that W may be read before the predecessor has finished).
+//
+// The same kernel with 128-row activation tiles (NB = 128, one CTA per SM) takes the products of small models whose tiles
+// leave most SMs idle: 360 x 1024 outputs are 24 tiles of 128 x 128.
 //
 // Warp 0: TMA producer; warp 1: TMEM, MMA issue; warps 2-5: accumulator -> shared memory; all warps: reduction over
 // the cluster and epilogue.  Every wait is bounded (common.cuh).
@@ -31,14 +34,14 @@ struct SkinnySmem {
   static constexpr int W_BYTES = SK_BM * SK_BK * 2;
   static constexpr int X_BYTES = NB * SK_BK * 2;
   static constexpr int STAGE = W_BYTES + X_BYTES;
-  static constexpr int STAGES = NB <= 16 ? 6 : NB <= 32 ? 5 : 4;
+  static constexpr int STAGES = NB <= 16 ? 6 : NB <= 32 ? 5 : NB <= 64 ? 4 : 6;
   static constexpr int TOTAL = STAGES * STAGE + 1024;
   static_assert(STAGES * STAGE >= NB * SK_BM * 4, "the partial tile reuses the ring");
-  static_assert(2 * (TOTAL + 1024) <= 227 * 1024, "two CTAs per SM");
+  static_assert(TOTAL <= 226 * 1024 && (NB > 64 || 2 * (TOTAL + 1024) <= 227 * 1024), "two CTAs per SM up to 64 rows");
 };
 
 template <int NB>
-__global__ void __launch_bounds__(SK_THREADS, 2)
+__global__ void __launch_bounds__(SK_THREADS, NB > 64 ? 1 : 2)
 skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                    const SkinnyArgs p) {
   using S = SkinnySmem<NB>;
@@ -49,7 +52,10 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   constexpr uint32_t TMEM_COLS = NB < 32 ? 32 : NB;
-  const int rank = (int)blockIdx.x % p.splits, tile = (int)blockIdx.x / p.splits;
+  const int rank = (int)blockIdx.x % p.splits;
+  const int tile = (int)blockIdx.x / p.splits % p.num_n;       // of W
+  const int m0 = (int)blockIdx.x / p.splits / p.num_n * NB;    // first activation row
+  const int rows = min(NB, p.M - m0);
   const int kb0 = rank * p.kb_per_cta;
   const int n_kb = min(p.kb_per_cta, p.num_kb - kb0);      // >= 1: the host leaves no CTA of a cluster without work
 
@@ -91,7 +97,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         }
       };
       auto load_x = [&](int i, int stage) {
-        tma_load_2d(smem_base + stage * S::STAGE + S::W_BYTES, &tmX, smem_u32(&bar_full[stage]), (kb0 + i) * SK_BK, 0);
+        tma_load_2d(smem_base + stage * S::STAGE + S::W_BYTES, &tmX, smem_u32(&bar_full[stage]), (kb0 + i) * SK_BK, m0);
       };
       const int head = p.w_static ? min(n_kb, S::STAGES) : 0;
       for (int i = 0; i < head; ++i) load_w(i, i);           // the ring's first turn: every stage is free
@@ -131,7 +137,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       tc_fence_after();
       const uint32_t dst = smem_base + (quad * 32 + lane) * 4;
 #pragma unroll 1
-      for (int c = 0; c < NB && c < p.M; c += 16) {
+      for (int c = 0; c < NB && c < rows; c += 16) {
         uint32_t r[16];
         __syncwarp();
         tmem_ld_32x16(tmem_base + c + (static_cast<uint32_t>(quad * 32) << 16), r);
@@ -152,12 +158,13 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   // ---------------------------------------------------------------- sum over the cluster, epilogue: 4 columns a thread
   const int cols = p.act == 3 ? SK_BM / 2 : SK_BM;           // output columns of the tile
   const int per_row = cols / 4;
-  for (int u = rank * SK_THREADS + (int)threadIdx.x; u < p.M * per_row; u += p.splits * SK_THREADS) {
-    const int m = u / per_row, f = (u - m * per_row) * 4;
+  for (int u = rank * SK_THREADS + (int)threadIdx.x; u < rows * per_row; u += p.splits * SK_THREADS) {
+    const int r = u / per_row, f = (u - r * per_row) * 4;
+    const long long m = m0 + r;
     const int col = tile * cols + f;
     if (col >= p.N) continue;
     auto total = [&](int feature) {
-      const uint32_t off = smem_base + (m * SK_BM + feature) * 4;
+      const uint32_t off = smem_base + (r * SK_BM + feature) * 4;
       float4 x[8];                      // every load in flight before the first addition
 #pragma unroll
       for (int s = 0; s < 8; ++s)
@@ -192,7 +199,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
     if (p.residual) {
-      const __nv_bfloat16* rp = p.residual + (long long)m * p.ldr + col;
+      const __nv_bfloat16* rp = p.residual + m * p.ldr + col;
       if (whole) {
         const uint2 b = *reinterpret_cast<const uint2*>(rp);
         v[0] += bf16_lo(b.x); v[1] += bf16_hi(b.x); v[2] += bf16_lo(b.y); v[3] += bf16_hi(b.y);
@@ -201,14 +208,14 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
     if (p.out_fp32) {
-      float* op = reinterpret_cast<float*>(p.out) + (long long)m * p.ldo + col;
+      float* op = reinterpret_cast<float*>(p.out) + m * p.ldo + col;
       if (whole) {
         if (DZ_STORE_OK(op, 16)) *reinterpret_cast<float4*>(op) = make_float4(v[0], v[1], v[2], v[3]);
       } else {
         for (int j = 0; j < 4; ++j) if (col + j < p.N && DZ_STORE_OK(op + j, 4)) op[j] = v[j];
       }
     } else {
-      __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.out) + (long long)m * p.ldo + col;
+      __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.out) + m * p.ldo + col;
       if (whole) {
         if (DZ_STORE_OK(op, 8))
           *reinterpret_cast<uint2*>(op) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
@@ -229,7 +236,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
 }
 
-static int sk_nb(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : 64; }
+static int sk_nb(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
 
 int skinny_map_w(CUtensorMap* map, const void* W, long long ldw, int rows, int K, bool swiglu) {
   return make_tmap_bf16_2d(map, W, rows, K, ldw, swiglu ? SK_BM / 2 : SK_BM, SK_BK, true);
@@ -243,6 +250,7 @@ int skinny_map_x(CUtensorMap* map, const void* A, long long lda, int M, int K) {
 // 8192 (16 tiles) 30.5 / 18.4 / 12.1 / 10.6 with 1 / 2 / 4 / 8 CTAs a tile; N 12288 K 4096 (96 tiles) 22.2 / 20.0 / 26.0
 // with 1 / 2 / 3; N 6144 K 2048 (48 tiles) 8.7 / 13.1 with 4 / 6; N 20480 K 5120 (160 tiles) 36.5 / 43.5 with 1 / 2.
 // A launch of a dependent chain keeps to one CTA per SM, so that the next launch fits beside it and can fill its ring.
+// (For 128-row tiles the caller chooses: split_pays in block_forward.cu.)
 static int choose_splits(int tiles, int num_kb, bool dependent) {
   int s = (dependent ? sm_count() : 256) / (tiles > 0 ? tiles : 1);
   if (s > num_kb / 3) s = num_kb / 3;
@@ -263,16 +271,21 @@ static int launch_nb(const CUtensorMap& tmW, const CUtensorMap& tmX, const Skinn
 int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, int splits, bool dependent,
                   cudaStream_t stream) {
   const int cols = a.act == 3 ? SK_BM / 2 : SK_BM;
-  const int tiles = (a.N + cols - 1) / cols;
+  const int nb = sk_nb(a.M);
+  a.num_n = (a.N + cols - 1) / cols;
+  const long long tiles_ll = (long long)a.num_n * ((a.M + nb - 1) / nb);
+  if (tiles_ll * 8 > 0x7fffffffLL) return DZ_ERR_TOO_LARGE;
+  const int tiles = (int)tiles_ll;
   a.num_kb = (a.K + SK_BK - 1) / SK_BK;
   if (splits <= 0) splits = choose_splits(tiles, a.num_kb, dependent);
   if (splits > 8) splits = 8;
   a.kb_per_cta = (a.num_kb + splits - 1) / splits;
   a.splits = (a.num_kb + a.kb_per_cta - 1) / a.kb_per_cta;     // no CTA without a K block
-  switch (sk_nb(a.M)) {
+  switch (nb) {
     case 16: return launch_nb<16>(tmW, tmX, a, tiles, dependent, stream);
     case 32: return launch_nb<32>(tmW, tmX, a, tiles, dependent, stream);
-    default: return launch_nb<64>(tmW, tmX, a, tiles, dependent, stream);
+    case 64: return launch_nb<64>(tmW, tmX, a, tiles, dependent, stream);
+    default: return launch_nb<128>(tmW, tmX, a, tiles, dependent, stream);
   }
 }
 
@@ -281,13 +294,12 @@ int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, 
 using namespace dz;
 DZ_DEBUG_TU(skinny)
 
-// Same contract as dz_gemm_bf16_tn (gemm_sm100.cu) for M <= 64; act 3: W = gate rows | up rows (N each), out [M, N] =
+// Same contract as dz_gemm_bf16_tn (gemm_sm100.cu); act 3: W = gate rows | up rows (N each), out [M, N] =
 // silu(A gate^T) * (A up^T), bf16, without bias, residual or scale.  splits: 0 = choose, else CTAs per tile (1 to 8).
 extern "C" int dz_gemm_skinny(const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo,
                               const void* bias, const void* residual, long long ldr, int M, int N, int K, int act,
                               int out_fp32, float out_scale, int splits, uint32_t* err, cudaStream_t stream) {
   if (!A || !W || !out || M <= 0 || N <= 0 || K <= 0 || act < 0 || act > 3 || splits < 0) return DZ_ERR_ARG;
-  if (M > SK_MAX_ROWS) return DZ_ERR_TOO_LARGE;
   if ((K & 7) || (lda & 7) || (ldw & 7)) return DZ_ERR_ALIGN;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(W) & 15)) return DZ_ERR_ALIGN;
   const int esz = out_fp32 ? 4 : 2;

@@ -19,7 +19,7 @@ def _close(y, ref, K):
     assert err < (2.0 ** -8 if y.dtype == torch.bfloat16 else 0.0) + 16 * K ** 0.5 * 2.0 ** -24, err
 
 
-@pytest.mark.parametrize("M", [1, 16, 17, 64])
+@pytest.mark.parametrize("M", [1, 16, 17, 64, 65, 128, 300])
 @pytest.mark.parametrize("N,K", [(8, 8), (128, 64), (200, 72), (2048, 2048), (1032, 8200), (25000, 136)])
 @pytest.mark.parametrize("splits", [0, 1, 3, 8])
 def test_skinny_gemm(M, N, K, splits):
