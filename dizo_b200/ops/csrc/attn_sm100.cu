@@ -34,24 +34,31 @@ constexpr int A_THREADS = 320;
 constexpr int A_KV_STAGES = 2;
 constexpr float A_RESCALE_THRESHOLD = 8.0f;  // log2 units
 
-template <int HDP>
+template <int HDP, int NT>
 struct AttnSmem {
   static constexpr int Q_TILE = A_BQ * HDP * 2;     // per query tile
   static constexpr int KV_TILE = A_BKV * HDP * 2;   // per K or V stage
   static constexpr int OFF_Q = 0;
-  static constexpr int OFF_K = OFF_Q + 2 * Q_TILE;
+  static constexpr int OFF_K = OFF_Q + NT * Q_TILE;
   static constexpr int OFF_V = OFF_K + A_KV_STAGES * KV_TILE;
   static constexpr int USED = OFF_V + A_KV_STAGES * KV_TILE + 1024;
-  // at least 120 KB so that two CTAs (each wanting all 512 TMEM columns) never share an SM
-  static constexpr int TOTAL = USED < 120 * 1024 ? 120 * 1024 : USED;
+  // two tiles: at least 120 KB so that two CTAs (each wanting all 512 TMEM columns) never share an SM; one tile takes 256
+  // columns and two CTAs fit in both respects
+  static constexpr int TOTAL = NT == 2 && USED < 120 * 1024 ? 120 * 1024 : USED;
 };
 
-template <int HDP>
-__global__ void __launch_bounds__(A_THREADS, 1)
+// NT: query tiles per CTA.  2: they ping-pong (above).  1: sequences of at most 128 queries, which have no second tile: a
+// CTA of 6 warps with 82 KB and 256 TMEM columns at head dim <= 64, so that two share an SM and one's loads run beside the
+// other's softmax.  Two tiles / one, us: 16 x 120 tokens, 32 heads of 64 23.7 / 13.6; 16 x 64 tokens, 12 heads 12.0 / 7.4;
+// 8 x 48 tokens, 16 heads (one round of CTAs either way) 7.2 / 7.0.
+template <int HDP, int NT>
+__global__ void __launch_bounds__(NT == 2 ? A_THREADS : 192, NT == 2 ? 1 : 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmKV,
                 const __grid_constant__ CUtensorMap tmPK, const __grid_constant__ CUtensorMap tmPV,
                 const AttnArgs p) {
-  using S = AttnSmem<HDP>;
+  using S = AttnSmem<HDP, NT>;
+  constexpr int W_MMA = 4 * NT, W_TMA = W_MMA + 1;      // warps
+  constexpr uint32_t TMEM_COLS = NT * 256;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_q;
   __shared__ __align__(8) uint64_t bar_k_full[A_KV_STAGES], bar_k_empty[A_KV_STAGES];
@@ -65,7 +72,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
 
   // Heaviest (latest) query tiles first: they have the most key blocks under causality.
-  const int pairs = (p.L + 2 * A_BQ - 1) / (2 * A_BQ);
+  const int pairs = (p.L + NT * A_BQ - 1) / (NT * A_BQ);
   const int pair = pairs - 1 - blockIdx.x;
   const int h = blockIdx.y;
   const int b = blockIdx.z;
@@ -75,8 +82,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   // Tile t covers query rows [q0[t], q0[t] + 128).  Block range of keys: [jb, nb[t]).
   int q0[2], nb[2], nvb[2];
-  q0[0] = pair * 2 * A_BQ;
-  q0[1] = q0[0] + A_BQ;
+  q0[0] = pair * NT * A_BQ;
+  q0[1] = NT == 2 ? q0[0] + A_BQ : p.L;        // a single tile: the second does not exist
   const int jb = min(pad, q0[0]) / A_BKV;  // first block that can hold a visible key
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
@@ -107,19 +114,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     fence_mbar_init();
   }
-  if (warp == 8) {
-    tmem_alloc(smem_u32(&s_tmem_base), 512);
+  if (warp == W_MMA) {
+    tmem_alloc(smem_u32(&s_tmem_base), TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
-  // TMEM columns: S0/P0 [0,128) S1/P1 [128,256) O0 [256,256+HDP) O1 [384,384+HDP)
+  // TMEM columns: S0/P0 [0,128) S1/P1 [128,256) O0 [256,256+HDP) O1 [384,384+HDP); one tile: S0/P0 [0,128) O0 [128,..)
   const uint32_t tm_s[2] = {tmem_base + 0u, tmem_base + 128u};
-  const uint32_t tm_o[2] = {tmem_base + 256u, tmem_base + 384u};
+  const uint32_t tm_o[2] = {tmem_base + NT * 128u, tmem_base + 384u};
 
-  if (warp == 9) {
+  if (warp == W_TMA) {
     if (lane == 0 && nvb_max > 0) {
       // ---------------------------------------------- TMA producer (one thread)
       const int row_base = b * p.L;
@@ -158,7 +165,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       }
     }
-  } else if (warp == 8) {
+  } else if (warp == W_MMA) {
     if (lane == 0 && nvb_max > 0) {
       // ---------------------------------------------- MMA issuer (one thread)
       bool ok = true;
@@ -169,7 +176,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // the descriptors are built once and each MMA adds a constant to their address field, so that issuing
       // stays cheaper than executing (building them per MMA took about 90 cycles each).
       const uint64_t q_desc0 = umma_desc_k_sw128(smem_base + S::OFF_Q);
-      const uint64_t q_desc1 = umma_desc_k_sw128(smem_base + S::OFF_Q + S::Q_TILE);
+      const uint64_t q_desc1 = umma_desc_k_sw128(smem_base + S::OFF_Q + (NT - 1) * S::Q_TILE);
       const uint64_t k_desc0 = umma_desc_k_sw128(smem_base + S::OFF_K);
       const uint64_t k_desc1 = umma_desc_k_sw128(smem_base + S::OFF_K + S::KV_TILE);
       const uint64_t v_desc0 = umma_desc_mn_sw128(smem_base + S::OFF_V, A_BKV * 128, 1024);
@@ -203,7 +210,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (ok) ok = mbar_wait(smem_u32(&bar_k_full[0]), 0, &s_abort, p.err, ERR_WAIT_FULL);
       if (ok) {
         tc_fence_after();
-        for (int t = 0; t < 2; ++t)
+        for (int t = 0; t < NT; ++t)
           if (nvb[t] > 0) issue_s(t, 0);
         umma_commit(smem_u32(&bar_k_empty[0]));
       }
@@ -219,7 +226,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                          ERR_WAIT_FULL);
           if (!ok) break;
         }
-        for (int t = 0; t < 2 && ok; ++t) {
+        for (int t = 0; t < NT && ok; ++t) {
           if (vb < nvb[t]) {
             ok = mbar_wait(smem_u32(&bar_p[t]), vb & 1, &s_abort, p.err, ERR_WAIT_MISC);
             if (!ok) break;
@@ -236,7 +243,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else {
     // ------------------------------------------------------------ softmax warpgroups
-    const int t = warp >> 2;           // query tile of this warpgroup
+    const int t = NT == 2 ? warp >> 2 : 0;   // query tile of this warpgroup
     const int quad = warp & 3;         // TMEM lane quadrant
     const int r = quad * 32 + lane;    // row inside the tile
     const int qi = q0[t] + r;          // query index inside the sequence
@@ -355,26 +362,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) {
+  if (warp == W_MMA) {
     __syncwarp();
     if (s_abort) {
       for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     }
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
-template <int HDP>
+template <int HDP, int NT>
 static int launch_attn(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const CUtensorMap& tmPK,
                        const CUtensorMap& tmPV, const AttnArgs& a, cudaStream_t stream) {
-  using S = AttnSmem<HDP>;
-  auto kern = attn_fwd_kernel<HDP>;
+  using S = AttnSmem<HDP, NT>;
+  auto kern = attn_fwd_kernel<HDP, NT>;
   static PerDeviceFlag configured;
   if (int rc_cfg = ensure_dyn_smem(configured, kern, S::TOTAL)) return rc_cfg;
-  int pairs = (a.L + 2 * A_BQ - 1) / (2 * A_BQ);
+  int pairs = (a.L + NT * A_BQ - 1) / (NT * A_BQ);
   dim3 grid(pairs, a.H, a.B);
-  kern<<<grid, A_THREADS, S::TOTAL, stream>>>(tmQ, tmKV, tmPK, tmPV, a);
+  kern<<<grid, NT == 2 ? A_THREADS : 192, S::TOTAL, stream>>>(tmQ, tmKV, tmPK, tmPV, a);
   return cuda_rc(cudaGetLastError());
 }
 
@@ -420,8 +427,9 @@ extern "C" int dz_attn_fwd_lse(const void* qkv, long long ld_qkv, int q_col0, in
   a.out = (__nv_bfloat16*)out; a.pad_left = pad_left; a.lse = lse;
   a.scale_log2 = scale * 1.4426950408889634f;
   a.q_col0 = q_col0; a.k_col0 = k_col0; a.v_col0 = v_col0; a.err = err;
-  if (hdp == 64) return launch_attn<64>(tmQ, tmKV, tmPK, tmPV, a, stream);
-  return launch_attn<128>(tmQ, tmKV, tmPK, tmPV, a, stream);
+  if (hdp == 64 && L <= A_BQ) return launch_attn<64, 1>(tmQ, tmKV, tmPK, tmPV, a, stream);
+  if (hdp == 64) return launch_attn<64, 2>(tmQ, tmKV, tmPK, tmPV, a, stream);
+  return launch_attn<128, 2>(tmQ, tmKV, tmPK, tmPV, a, stream);
 }
 
 extern "C" int dz_attn_fwd(const void* qkv, long long ld_qkv, int q_col0, int k_col0, int v_col0,
