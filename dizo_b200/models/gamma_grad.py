@@ -84,10 +84,11 @@ class _Replicated:
     def dgrad(self, w, which, dy, mask=None, residual=None):
         return bw.linear_dgrad(dy, self._wb(w, which)[0], mask=mask, residual=residual)
 
-    def x_delta(self, w, names, x):
-        """X (theta - theta_0)^T for the named constrained [d, d] weights of layer w.i: fp32 [M, d] each."""
+    def delta_dots(self, w, names, x, dys, outs):
+        """<dY, X (theta - theta_0)^T> for the named constrained [d, d] weights of layer w.i, into ``outs``."""
         ar = self.m.arena
-        return [gemm.linear(x, bw.diff(ar.view(n), ar.anchor_view(n)), out_dtype=torch.float32) for n in names]
+        for n, dy, out in zip(names, dys, outs):
+            bw.linear_dot(x, bw.diff(ar.view(n), ar.anchor_view(n)), dy, out=out)
 
 
 class _FSDP:
@@ -133,7 +134,7 @@ class _FSDP:
         K = segs[0]["w_shard"].shape[1]
         return bw.linear_dgrad(dy, self._gather(segs, N, K), mask=mask, residual=residual)
 
-    def x_delta(self, w, names, x):
+    def delta_dots(self, w, names, x, dys, outs):
         m, ar = self.m, self.m.arena
         d = m.config.hidden_size
         segs = []
@@ -141,7 +142,8 @@ class _FSDP:
             delta = bw.diff(ar.view(n).contiguous(), ar.anchor_view(n).contiguous())
             segs.append(dict(w_shard=delta, dst_row0=j * d + m.r * delta.shape[0]))
         t = gemm.linear(x, self._gather(segs, len(names) * d, d), out_dtype=torch.float32)
-        return [t[:, j * d:(j + 1) * d] for j in range(len(names))]
+        for j, (dy, out) in enumerate(zip(dys, outs)):
+            bw.dot(t[:, j * d:(j + 1) * d], dy, out=out)
 
 
 class GammaGrad:
@@ -241,9 +243,8 @@ class GammaGrad:
                 cols.append(j)
         if not names:
             return
-        for full, j, t in zip(names, cols, self.prov.x_delta(w, names, x1)):
-            s = self.slot_of[full]
-            bw.dot(t, dqkv[:, j * d:(j + 1) * d], out=grad[s:s + 1])
+        slots = [self.slot_of[full] for full in names]
+        self.prov.delta_dots(w, names, x1, [dqkv[:, j * d:(j + 1) * d] for j in cols], [grad[s:s + 1] for s in slots])
 
     # ------------------------------------------------------------------ main entry
     @torch.no_grad()

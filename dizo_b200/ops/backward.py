@@ -125,6 +125,29 @@ def dot(a: torch.Tensor, b: torch.Tensor, scale: float = 1.0, out: torch.Tensor 
     return out
 
 
+def linear_dot(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, scale: float = 1.0,
+               out: torch.Tensor | None = None) -> torch.Tensor:
+    """scale * sum((x @ w.T) * b): x [M, K], w [N, K], b [M, N] bf16 (row strides free); fp32 [1].  Where the two-SM GEMM
+    runs, its epilogue takes the inner product with the fp32 accumulators and the [M, N] product is never stored."""
+    from . import gemm
+    M, N = x.shape[0], w.shape[0]
+    fused = (x.is_cuda and M >= 256 and ((M + 255) // 256) * ((N + 255) // 256) >= 48 and b.stride(1) == 1
+             and b.stride(0) % 8 == 0 and b.data_ptr() % 16 == 0 and gemm._VARIANT in (0, 2))
+    if not fused:
+        return dot(gemm.linear(x, w, out_dtype=torch.float32), b, scale=scale, out=out)
+    assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
+    assert b.shape == (M, N) and w.shape[1] == x.shape[1] and x.stride(1) == 1 and w.stride(1) == 1
+    L = _lib.lib()
+    partials = torch.empty(L.dz_gemm2_dot_partials(M, N), dtype=torch.float32, device=x.device)
+    if out is None:
+        out = torch.empty(1, dtype=torch.float32, device=x.device)
+    rc = L.dz_gemm2_dot(_lib.ptr(x), ll(x.stride(0)), _lib.ptr(w), ll(w.stride(0)), _lib.ptr(b), ll(b.stride(0)), M, N,
+                        x.shape[1], ctypes.c_float(scale), _lib.ptr(partials), _lib.ptr(out),
+                        _lib.ptr(_lib.err_word(x.device)), _lib.stream_ptr())
+    _lib.check(rc, "dz_gemm2_dot")
+    return out
+
+
 def scatter_rows(src: torch.Tensor, idx: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
     """dst[idx[r], :] = src[r, :] (rows of ``idx`` distinct)."""
     if not src.is_cuda:

@@ -384,6 +384,13 @@ extern "C" int dz_dot_f32_bf16(const float* a, long long lda, const void* b, lon
   return cuda_rc(cudaGetLastError());
 }
 
+// *out = scale * sum of n partial sums, in a fixed order
+extern "C" int dz_dot_final(const float* partials, int n, float scale, float* out, cudaStream_t stream) {
+  if (!partials || !out || n <= 0) return DZ_ERR_ARG;
+  dot_final_kernel<<<1, 256, 0, stream>>>(partials, n, scale, out);
+  return cuda_rc(cudaGetLastError());
+}
+
 // dst[idx[r], :] = src[r, :]
 extern "C" int dz_scatter_rows(const void* src, long long lds, const int* idx, void* dst, long long ldd,
                                long long rows, int d, long long n_dst, cudaStream_t stream) {

@@ -56,6 +56,8 @@ struct Gemm2Args {
   int wide_mask;            // the mask rows are 16-byte aligned
   const float* rope_cs;     // fp32 [n_pos][64][2] = (cos, sin)
   int rope_L, rope_pos0, rope_n_pos, rope_H, rope_Hkv;
+  // act 5: nothing of the product is stored; sum(product * residual) of each tile, by epilogue warp
+  float* dot_partials;      // [num_m * num_n][8]
 };
 
 __device__ __forceinline__ void tile_coords2(int tile, const Gemm2Args& p, int& mb, int& nb) {
@@ -263,6 +265,41 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             store32(head_out, n_rep, 64 + pc * 32, hi);
           }
         }
+      } else if (p.act == 5) {
+        // <A W^T, residual>: this lane's row of the tile against the row of the residual, the accumulators in fp32
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+        for (int c = 0; c < p.bn / 32; ++c) {
+          uint32_t r[32];
+          __syncwarp();                                   // lanes of rows past M skipped the sums above
+          tmem_ld_32x32(t_row + c * 32, r);
+          tmem_ld_wait();
+          const int col0 = nb * p.bn + c * 32;
+          if (!row_ok || col0 >= p.N) continue;
+          const __nv_bfloat16* rp = p.residual + row * p.ldr + col0;
+          if (col0 + 32 <= p.N) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint4 b = __ldg(reinterpret_cast<const uint4*>(rp) + q);
+              const uint32_t w[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                s[j] = fmaf(__uint_as_float(r[q * 8 + 2 * j]), bf16_lo(w[j]), s[j]);
+                s[j] = fmaf(__uint_as_float(r[q * 8 + 2 * j + 1]), bf16_hi(w[j]), s[j]);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (col0 + j < p.N) s[j & 3] = fmaf(__uint_as_float(r[j]), __bfloat162float(rp[j]), s[j & 3]);
+          }
+        }
+        __syncwarp();
+        float t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+        float* pp = p.dot_partials + (long long)tile * 8 + rank * 4 + quad;
+        if (lane == 0 && DZ_STORE_OK(pp, 4)) *pp = t;
       } else if (p.act == 3) {
         // out[row, nb * 128 + j] = silu(gate_j) * up_j from the fp32 accumulators, one rounding to bf16
 #pragma unroll 1
@@ -446,6 +483,8 @@ struct Gemm2Extra {
   const void* mask;         // ReLU backward (MN-major form)
   long long ldm;
   const Gemm2Args* rope;    // act 4
+  float* dot_partials;      // act 5
+  int* dot_n;               // act 5: receives the number of partial sums
 };
 
 template <bool B_MN>
@@ -475,7 +514,7 @@ extern "C" int dz_gemm2_bf16_tn(const void* A, long long lda, const void* W, lon
                                 long long ldo, const void* bias, const void* residual, long long ldr,
                                 int M, int N, int K, int act, int out_fp32, float out_scale,
                                 uint32_t* err, cudaStream_t stream) {
-  if (act == 4) return DZ_ERR_ARG;
+  if (act >= 4) return DZ_ERR_ARG;
   return gemm2_launch<false>(A, lda, W, ldw, out, ldo, bias, residual, ldr, M, N, K, act, out_fp32, out_scale, err,
                              stream, Gemm2Extra{});
 }
@@ -489,6 +528,29 @@ extern "C" int dz_gemm2_bf16_nn(const void* A, long long lda, const void* W, lon
   Gemm2Extra x{};
   x.mask = mask; x.ldm = ldm;
   return gemm2_launch<true>(A, lda, W, ldw, out, ldo, nullptr, residual, ldr, M, N, K, 0, out_fp32, 1.0f, err, stream, x);
+}
+
+extern "C" int dz_dot_final(const float* partials, int n, float scale, float* out, cudaStream_t stream);
+
+// *out = scale * sum((A W^T) * D) for D [M, ldd] bf16: the product is reduced tile by tile in the epilogue and never
+// stored.  partials: fp32 scratch of dz_gemm2_dot_partials(M, N) elements.  Fixed order: bitwise reproducible.
+extern "C" int dz_gemm2_dot_partials(int M, int N) {
+  const long long n = (long long)((M + G2_BM - 1) / G2_BM) * ((N + 223) / 224) * 8;
+  return n > 0x7fffffffLL ? 0 : (int)n;
+}
+extern "C" int dz_gemm2_dot(const void* A, long long lda, const void* W, long long ldw, const void* D, long long ldd,
+                            int M, int N, int K, float scale, float* partials, float* out, uint32_t* err,
+                            cudaStream_t stream) {
+  if (!D || !partials || !out) return DZ_ERR_ARG;
+  Gemm2Extra x{};
+  int n = 0;
+  x.dot_partials = partials;
+  x.dot_n = &n;
+  // the product itself has no destination: D stands in for the alignment checks of one
+  int rc = gemm2_launch<false>(A, lda, W, ldw, const_cast<void*>(D), ldd, nullptr, D, ldd, M, N, K, 5, 0, 1.0f, err, stream,
+                               x);
+  if (rc) return rc;
+  return dz_dot_final(partials, n, scale, out, stream);
 }
 
 // Fused q | k | v projection with the rotary embedding in the epilogue: A [M, K], W [(H + 2 Hkv) * 128, K] ->
@@ -560,7 +622,7 @@ static int gemm2_launch(const void* A, long long lda, const void* W, long long l
     max_clusters = n < sm_count() / 2 ? n : sm_count() / 2;
   }
   a.num_m = (M + G2_BM - 1) / G2_BM;
-  a.bn = act >= 3 || B_MN ? G2_BN : gemm2_tile_n(a.num_m, N, max_clusters);
+  a.bn = act == 3 || act == 4 || B_MN ? G2_BN : gemm2_tile_n(a.num_m, N, max_clusters);
   a.num_n = (N + a.bn - 1) / a.bn;
   // M tiles per rasterisation group: a group's A tiles stay in L2 while its W tiles stream once
   static const int group_env = [] { const char* e = getenv("DIZO_GEMM_GROUP_M"); return e ? atoi(e) : 0; }();
@@ -577,6 +639,8 @@ static int gemm2_launch(const void* A, long long lda, const void* W, long long l
             : make_tmap_bf16_2d(&tmB, W, N, K, ldw, a.bn / 2, G2_BK, true);
   if (rc) return rc;
   const int tiles = a.num_m * a.num_n;
+  a.dot_partials = extra.dot_partials;
+  if (extra.dot_n) *extra.dot_n = tiles * 8;
   int clusters = max_clusters;
   if (tiles < clusters) clusters = tiles;
   gemm2_bf16_kernel<B_MN><<<clusters * 2, G2_THREADS, G2_SMEM, stream>>>(tmA, tmB, a);

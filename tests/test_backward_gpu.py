@@ -244,3 +244,22 @@ def test_gamma_grad_kernel_backward_other_layouts(variant):
     assert abs(loss.item() - ref_loss.item()) < 3e-2 * max(1.0, abs(ref_loss.item()))
     cos = torch.nn.functional.cosine_similarity(grad, a.grad.float(), dim=0).item()
     assert cos > 0.97, (cos, grad, a.grad)
+
+
+@pytest.mark.parametrize("M,N,K", [(4096, 2560, 2560), (3000, 1000, 136), (1400, 2552, 72), (300, 64, 64)])
+def test_linear_dot(M, N, K):
+    """The inner product taken in the GEMM epilogue (last shape: product stored, then reduced)."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(N, K, device=DEV, generator=g) * 0.05).bfloat16()
+    wide = torch.randn(M, 2 * N, device=DEV, generator=g).bfloat16()
+    b = wide[:, N:]
+    got = bw.linear_dot(x, w, b, scale=0.5)
+    again = bw.linear_dot(x, w, b, scale=0.5)
+    _sync_ok()
+    assert torch.equal(got, again)
+    prod = x.double() @ w.double().t()
+    want = 0.5 * (prod * b.double()).sum()
+    # fp32 products of K terms and a sum of M N of them: random signs, so 2^-24 of the root of the sum of squares, x 64
+    bound = 64 * 2.0 ** -24 * (x.double().pow(2).sum().sqrt() * w.double().pow(2).sum().sqrt() * b.double().abs().max())
+    assert (got.double() - want).abs() <= bound
