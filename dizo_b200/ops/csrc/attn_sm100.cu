@@ -24,6 +24,7 @@
 // tile while the other does its exps.
 #include "common.cuh"
 #include "host_util.h"
+#include "pdl.cuh"
 #include "attn_args.h"
 
 namespace dz {
@@ -76,27 +77,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int pair = pairs - 1 - blockIdx.x;
   const int h = blockIdx.y;
   const int b = blockIdx.z;
-  const int pad = p.pad_left ? p.pad_left[b] : 0;
   const int hd = p.hd;
   const int has_prefix = p.n_prefix > 0 ? 1 : 0;
-
-  // Tile t covers query rows [q0[t], q0[t] + 128).  Block range of keys: [jb, nb[t]).
-  int q0[2], nb[2], nvb[2];
-  q0[0] = pair * NT * A_BQ;
-  q0[1] = NT == 2 ? q0[0] + A_BQ : p.L;        // a single tile: the second does not exist
-  const int jb = min(pad, q0[0]) / A_BKV;  // first block that can hold a visible key
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    if (q0[t] < p.L) {
-      int last_row = min(q0[t] + A_BQ, p.L) - 1;
-      nb[t] = last_row / A_BKV + 1;
-      nvb[t] = has_prefix + nb[t] - jb;
-    } else {
-      nb[t] = jb;
-      nvb[t] = 0;  // tile does not exist
-    }
-  }
-  const int nvb_max = max(nvb[0], nvb[1]);
 
   if (threadIdx.x == 0) {
     s_abort = 0;
@@ -122,6 +104,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  pdl_trigger();
+  pdl_wait();
+  const int pad = p.pad_left ? p.pad_left[b] : 0;
+
+  // Tile t covers query rows [q0[t], q0[t] + 128).  Block range of keys: [jb, nb[t]).
+  int q0[2], nb[2], nvb[2];
+  q0[0] = pair * NT * A_BQ;
+  q0[1] = NT == 2 ? q0[0] + A_BQ : p.L;        // a single tile: the second does not exist
+  const int jb = min(pad, q0[0]) / A_BKV;  // first block that can hold a visible key
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    if (q0[t] < p.L) {
+      int last_row = min(q0[t] + A_BQ, p.L) - 1;
+      nb[t] = last_row / A_BKV + 1;
+      nvb[t] = has_prefix + nb[t] - jb;
+    } else {
+      nb[t] = jb;
+      nvb[t] = 0;  // tile does not exist
+    }
+  }
+  const int nvb_max = max(nvb[0], nvb[1]);
+
   // TMEM columns: S0/P0 [0,128) S1/P1 [128,256) O0 [256,256+HDP) O1 [384,384+HDP); one tile: S0/P0 [0,128) O0 [128,..)
   const uint32_t tm_s[2] = {tmem_base + 0u, tmem_base + 128u};
   const uint32_t tm_o[2] = {tmem_base + NT * 128u, tmem_base + 384u};
@@ -381,8 +385,7 @@ static int launch_attn(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const CU
   if (int rc_cfg = ensure_dyn_smem(configured, kern, S::TOTAL)) return rc_cfg;
   int pairs = (a.L + NT * A_BQ - 1) / (NT * A_BQ);
   dim3 grid(pairs, a.H, a.B);
-  kern<<<grid, NT == 2 ? A_THREADS : 192, S::TOTAL, stream>>>(tmQ, tmKV, tmPK, tmPV, a);
-  return cuda_rc(cudaGetLastError());
+  return cuda_rc(pdl_launch(kern, grid, NT == 2 ? A_THREADS : 192, S::TOTAL, stream, 1, true, tmQ, tmKV, tmPK, tmPV, a));
 }
 
 }  // namespace dz

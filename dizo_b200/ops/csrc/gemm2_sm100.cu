@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "cluster2sm.cuh"
 #include "host_util.h"
+#include "pdl.cuh"
 
 namespace dz {
 
@@ -120,6 +121,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   cluster_sync_all();          // peer barriers are initialised before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (each CTA)
@@ -280,7 +283,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           if (col0 + 32 <= p.N) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              const uint4 b = __ldg(reinterpret_cast<const uint4*>(rp) + q);
+              const uint4 b = reinterpret_cast<const uint4*>(rp)[q];
               const uint32_t w[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
@@ -371,7 +374,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             if (full_chunk && p.wide_mask) {
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
-                const uint4 b = __ldg(reinterpret_cast<const uint4*>(mp) + q);
+                const uint4 b = reinterpret_cast<const uint4*>(mp)[q];
                 const uint32_t w[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -392,7 +395,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 uint32_t b[8];
-                asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                              : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]),
                                "=r"(b[7])
                              : "l"(rp + h * 16));
@@ -406,7 +409,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
               const uint4* rp4 = reinterpret_cast<const uint4*>(rp);
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
-                uint4 b = __ldg(rp4 + q);
+                const uint4 b = rp4[q];
                 v[q * 8 + 0] += bf16_lo(b.x); v[q * 8 + 1] += bf16_hi(b.x);
                 v[q * 8 + 2] += bf16_lo(b.y); v[q * 8 + 3] += bf16_hi(b.y);
                 v[q * 8 + 4] += bf16_lo(b.z); v[q * 8 + 5] += bf16_hi(b.z);
@@ -643,6 +646,5 @@ static int gemm2_launch(const void* A, long long lda, const void* W, long long l
   if (extra.dot_n) *extra.dot_n = tiles * 8;
   int clusters = max_clusters;
   if (tiles < clusters) clusters = tiles;
-  gemm2_bf16_kernel<B_MN><<<clusters * 2, G2_THREADS, G2_SMEM, stream>>>(tmA, tmB, a);
-  return cuda_rc(cudaGetLastError());
+  return cuda_rc(pdl_launch(gemm2_bf16_kernel<B_MN>, dim3(clusters * 2), G2_THREADS, G2_SMEM, stream, 1, true, tmA, tmB, a));
 }

@@ -22,6 +22,7 @@
 // (large_models/ht_opt.py:956, large_models/trainer.py:1469-1489).
 #include "common.cuh"
 #include "host_util.h"
+#include "pdl.cuh"
 
 namespace dz {
 
@@ -119,6 +120,8 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = s_tmem_base;
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -270,7 +273,7 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 const uint4* rp4 = reinterpret_cast<const uint4*>(rp);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                  uint4 b = __ldg(rp4 + q);
+                  const uint4 b = rp4[q];
                   v[q * 8 + 0] += bf16_lo(b.x); v[q * 8 + 1] += bf16_hi(b.x);
                   v[q * 8 + 2] += bf16_lo(b.y); v[q * 8 + 3] += bf16_hi(b.y);
                   v[q * 8 + 4] += bf16_lo(b.z); v[q * 8 + 5] += bf16_hi(b.z);
@@ -376,8 +379,7 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmArgs&
   a.group_m = a.num_m < 16 ? a.num_m : 16;
   int tiles = a.num_m * a.num_n;
   int grid = tiles < sm_count() ? tiles : sm_count();
-  kern<<<grid, G_THREADS, S::TOTAL, stream>>>(tmA, tmB, a);
-  return cuda_rc(cudaGetLastError());
+  return cuda_rc(pdl_launch(kern, dim3(grid), G_THREADS, S::TOTAL, stream, 1, true, tmA, tmB, a));
 }
 
 static int check_common(const void* A, const void* W, int M, int N, int K, long long lda,

@@ -35,7 +35,7 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bf
   for (int i = 0; i < RMS_MAXV; ++i) {
     const int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
-      v[i] = xr[idx];
+      v[i] = __ldcg(xr + idx);
       const float f[8] = {bf16_lo(v[i].x), bf16_hi(v[i].x), bf16_lo(v[i].y), bf16_hi(v[i].y),
                           bf16_lo(v[i].z), bf16_hi(v[i].z), bf16_lo(v[i].w), bf16_hi(v[i].w)};
 #pragma unroll
@@ -149,7 +149,7 @@ extern "C" int dz_rmsnorm(const void* x, long long ldx, const void* w, void* y, 
   if (!x || !w || !y || rows <= 0 || d <= 0) return DZ_ERR_ARG;
   if ((d & 7) || (ldx & 7) || (ldy & 7) || !lk_al16(x) || !lk_al16(w) || !lk_al16(y)) return DZ_ERR_ALIGN;
   return rmsnorm_launch((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, ldy, rows, d, eps,
-                        false, stream);
+                        true, stream);
 }
 
 // in: bf16 [rows, ld_in] holding q (H*hd) | k (Hkv*hd) | v (Hkv*hd); out: bf16 [rows, ld_out] holding

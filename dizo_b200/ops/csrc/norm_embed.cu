@@ -35,7 +35,7 @@ layernorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
   for (int i = 0; i < LN_MAXV; ++i) {
     int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
-      v[i] = xr[idx];
+      v[i] = __ldcg(xr + idx);
       sum += bf16_lo(v[i].x) + bf16_hi(v[i].x) + bf16_lo(v[i].y) + bf16_hi(v[i].y) +
              bf16_lo(v[i].z) + bf16_hi(v[i].z) + bf16_lo(v[i].w) + bf16_hi(v[i].w);
     }
@@ -182,7 +182,7 @@ extern "C" int dz_layernorm(const void* x, long long ldx, const void* w, const v
   if ((d & 7) || (ldx & 7) || (ldy & 7) || !al16(x) || !al16(w) || !al16(b) || !al16(y))
     return DZ_ERR_ALIGN;
   return layernorm_launch((const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b,
-                          (__nv_bfloat16*)y, ldy, rows, d, eps, false, stream);
+                          (__nv_bfloat16*)y, ldy, rows, d, eps, true, stream);
 }
 
 extern "C" int dz_embed(const int* ids, const int* positions, const void* tok, long long ld_tok,

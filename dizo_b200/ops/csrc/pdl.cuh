@@ -4,6 +4,14 @@
 // predecessor has completed and its memory is visible, and because every kernel of such a chain waits before it
 // finishes, so has everything launched before it.  Both instructions do nothing in a kernel launched the ordinary way.
 //
+// Between its start and pdl_wait() a kernel shares the chip with its predecessors, so what they produce is never read with
+// non-coherent loads (ld.global.nc, __ldg): those are for weights and tables, complete many launches earlier.
+//
+// The GEMMs, the attention forward, the norms and the sweeps always launch this way (a kernel launched the ordinary way in
+// between serialises as before): the launch latency and the set-up of barriers, TMEM and tables run beside the predecessor's
+// tail.  OPT-125m training step 2.88 -> 2.55 ms, OPT-350m graph replay 3.97 -> 3.73, OPT-2.7b 44.5 -> 44.3, scoring with
+// OPT-1.3b 10.5 -> 10.0.
+//
 // A kernel that allocates TMEM triggers after its allocation: its dependents are then only resident beside CTAs that
 // already own their columns, so an allocation can never wait for a CTA that waits for it.
 #pragma once

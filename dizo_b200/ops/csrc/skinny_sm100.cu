@@ -249,10 +249,10 @@ int skinny_map_x(CUtensorMap* map, const void* A, long long lda, int M, int K) {
 // larger clusters do not pack beyond that) with at least three 64-wide K blocks each.  Measured at one row, us: N 2048 K
 // 8192 (16 tiles) 30.5 / 18.4 / 12.1 / 10.6 with 1 / 2 / 4 / 8 CTAs a tile; N 12288 K 4096 (96 tiles) 22.2 / 20.0 / 26.0
 // with 1 / 2 / 3; N 6144 K 2048 (48 tiles) 8.7 / 13.1 with 4 / 6; N 20480 K 5120 (160 tiles) 36.5 / 43.5 with 1 / 2.
-// A launch of a dependent chain keeps to one CTA per SM, so that the next launch fits beside it and can fill its ring.
+// A launch of a decoding step keeps to one CTA per SM, so that the next launch fits beside it and can fill its ring.
 // (For 128-row tiles the caller chooses: split_pays in block_forward.cu.)
-static int choose_splits(int tiles, int num_kb, bool dependent) {
-  int s = (dependent ? sm_count() : 256) / (tiles > 0 ? tiles : 1);
+static int choose_splits(int tiles, int num_kb, bool in_step) {
+  int s = (in_step ? sm_count() : 256) / (tiles > 0 ? tiles : 1);
   if (s > num_kb / 3) s = num_kb / 3;
   return s < 1 ? 1 : s > 8 ? 8 : s;
 }
@@ -277,7 +277,7 @@ int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, 
   if (tiles_ll * 8 > 0x7fffffffLL) return DZ_ERR_TOO_LARGE;
   const int tiles = (int)tiles_ll;
   a.num_kb = (a.K + SK_BK - 1) / SK_BK;
-  if (splits <= 0) splits = choose_splits(tiles, a.num_kb, dependent);
+  if (splits <= 0) splits = choose_splits(tiles, a.num_kb, a.w_static != 0);
   if (splits > 8) splits = 8;
   a.kb_per_cta = (a.num_kb + splits - 1) / splits;
   a.splits = (a.num_kb + a.kb_per_cta - 1) / a.kb_per_cta;     // no CTA without a K block
@@ -318,5 +318,5 @@ extern "C" int dz_gemm_skinny(const void* A, long long lda, const void* W, long 
   if (rc) return rc;
   rc = skinny_map_x(&tmX, A, lda, M, K);
   if (rc) return rc;
-  return skinny_launch(tmW, tmX, a, splits, false, stream);
+  return skinny_launch(tmW, tmX, a, splits, true, stream);
 }

@@ -27,6 +27,7 @@
 // (:581-584) and the apply/reverse projection passes (:405-451).
 #include "common.cuh"
 #include "host_util.h"
+#include "pdl.cuh"
 #include "philox.cuh"
 
 namespace dz {
@@ -232,10 +233,7 @@ zo_sweep_kernel(const ZoSweepArgs a_in) {
   constexpr int UNROLL = DUAL ? 2 : 4;              // 16-byte loads in flight per lane
   constexpr int TS = SMALL ? 2 : 7;                 // log2 bytes between table entries
   ZoSweepArgs a = a_in;
-  if (a.seed1_dev) {
-    a.seed1 = *a.seed1_dev;     // a captured launch takes the step's seed from memory,
-    if (SR) a.sr_seed = a.seed1 * 0x9E3779B97F4A7C15ull + 1ull;   // and its rounding stream follows the seed
-  }
+  pdl_trigger();
   extern __shared__ __align__(16) uint8_t zo_smem[];
   const char* tab;
   if (SMALL) {
@@ -246,10 +244,15 @@ zo_sweep_kernel(const ZoSweepArgs a_in) {
     gauss_table_to_smem(zo_smem, a.gauss_table, threadIdx.x, THREADS);
     tab = reinterpret_cast<const char*>(zo_smem) + 4 * (threadIdx.x & 31);   // this lane's bank
   }
+  pdl_wait();                   // the quantile table above is a constant; everything below may be the predecessor's
+  if (a.seed1_dev) {
+    a.seed1 = *a.seed1_dev;     // a captured launch takes the step's seed from memory,
+    if (SR) a.sr_seed = a.seed1 * 0x9E3779B97F4A7C15ull + 1ull;   // and its rounding stream follows the seed
+  }
   __syncthreads();
   float c1 = a.c1, c2 = a.c2;
-  if (a.c1_ptr) c1 *= __ldg(a.c1_ptr);
-  if (Z2 && a.c2_ptr) c2 *= __ldg(a.c2_ptr);
+  if (a.c1_ptr) c1 *= __ldcg(a.c1_ptr);
+  if (Z2 && a.c2_ptr) c2 *= __ldcg(a.c2_ptr);
   const uint32_t c1_pair = bf16x2_splat(c1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -265,7 +268,7 @@ zo_sweep_kernel(const ZoSweepArgs a_in) {
   ZoTensor t = a.table[cur];
   long long t_next = (cur + 1 < a.t_end) ? a.table[cur + 1].offset : (1ll << 62);
   float alpha = 1.f;
-  if (BLEND && t.slot >= 0) alpha = __ldg(a.alpha + t.slot);
+  if (BLEND && t.slot >= 0) alpha = __ldcg(a.alpha + t.slot);
   PhiloxStream zs = philox_stream(a.seed1, t.tensor_id, 0u), rs = zs;
   if (SR) rs = philox_stream(a.sr_seed, t.tensor_id, 1u);
 
@@ -278,7 +281,7 @@ zo_sweep_kernel(const ZoSweepArgs a_in) {
       while (cur + 1 < a.t_end && a.table[cur + 1].offset <= cpos) ++cur;
       t = a.table[cur];
       t_next = (cur + 1 < a.t_end) ? a.table[cur + 1].offset : (1ll << 62);
-      if (BLEND && t.slot >= 0) alpha = __ldg(a.alpha + t.slot);
+      if (BLEND && t.slot >= 0) alpha = __ldcg(a.alpha + t.slot);
       zs = philox_stream(a.seed1, t.tensor_id, 0u);
       if (SR) rs = philox_stream(a.sr_seed, t.tensor_id, 1u);
     }
@@ -488,8 +491,7 @@ static int launch_sweep(const ZoSweepArgs& a, cudaStream_t stream) {
   }
   long long blocks = (chunks + threads / 32 - 1) / (threads / 32);
   int grid = (int)(blocks < sm_count() ? blocks : sm_count());
-  kern<<<grid, threads, smem, stream>>>(a);
-  return cuda_rc(cudaGetLastError());
+  return cuda_rc(pdl_launch(kern, dim3(grid), threads, smem, stream, 1, true, a));
 }
 
 }  // namespace dz
