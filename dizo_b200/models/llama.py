@@ -33,6 +33,7 @@ from types import SimpleNamespace
 import torch
 
 from ..ops import attention as attn_ops
+from ..ops import block as block_ops
 from ..ops import gemm, norm
 from ..ops import llama as llama_ops
 from .opt import Batch, OPTModel, _arena_sort_key, adapter_param_specs
@@ -263,6 +264,20 @@ class LlamaModel(OPTModel):
         h = gemm.linear(ctx, w.out_w, residual=h)
         return self._mlp(h, w)
 
+    # ------------------------------------------------------------------ blocks as native calls
+    _BLOCK_NAMES = ("input_layernorm.weight", "self_attn.q_proj.weight", "self_attn.o_proj.weight",
+                    "post_attention_layernorm.weight", "mlp.gate_proj.weight", "mlp.down_proj.weight")
+    _BLOCK_FUSED = (("self_attn.q_proj.weight", "self_attn.k_proj.weight", "self_attn.v_proj.weight"),
+                    ("mlp.gate_proj.weight", "mlp.up_proj.weight"))
+
+    def _make_block_runner(self, batch):
+        cfg = self.config
+        B, L = batch.input_ids.shape
+        rope = llama_ops.rope_table(self.num_prefix + L, cfg.head_dim, cfg.rope_theta, self.device)
+        return block_ops.LlamaBlockRunner(B, L, cfg.hidden_size, cfg.ffn_dim, cfg.num_attention_heads,
+                                          cfg.num_key_value_heads, cfg.rms_norm_eps, self.num_prefix, rope, batch.pad_left,
+                                          self.device, gemm._ROPE_FUSED, gemm._SWIGLU_FUSED)
+
     # ------------------------------------------------------------------ one-token decoding
     def decode_embed(self, tokens, positions, get):
         return norm.embed(tokens.view(-1, 1), None, get(self.EMBED), None).view(-1, self.config.hidden_size)
@@ -290,3 +305,6 @@ class LlamaModel(OPTModel):
         return dict(F=cfg.ffn_dim, H=cfg.num_attention_heads, Hkv=cfg.num_key_value_heads, act=3, rms=True,
                     pre_norm=True, eps=cfg.rms_norm_eps,
                     rope=llama_ops.rope_table(n_pos, cfg.head_dim, cfg.rope_theta, self.device))
+
+
+LlamaModel._native_block_of = LlamaModel

@@ -621,39 +621,45 @@ class OPTModel:
         return h
 
     # ------------------------------------------------------------------ blocks as native calls
-    def _block_runner(self, batch: Batch) -> "block_ops.BlockRunner | None":
-        """Runs whole blocks of this forward natively; None where :meth:`_layer_forward` has to (CPU, adapters, another
-        architecture or layout, forwards that record the QKV activations)."""
-        cfg = self.config
+    # tensors of a block in the order of ``ops.block.WEIGHTS``; the first of adjacent ones stands for the fused operand
+    _BLOCK_NAMES = ("self_attn_layer_norm.weight", "self_attn_layer_norm.bias", "self_attn.q_proj.weight",
+                    "self_attn.q_proj.bias", "self_attn.out_proj.weight", "self_attn.out_proj.bias",
+                    "final_layer_norm.weight", "final_layer_norm.bias", "fc1.weight", "fc1.bias", "fc2.weight", "fc2.bias")
+    _BLOCK_FUSED = (("self_attn.q_proj.weight", "self_attn.k_proj.weight", "self_attn.v_proj.weight"),
+                    ("self_attn.q_proj.bias", "self_attn.k_proj.bias", "self_attn.v_proj.bias"))
+
+    def _block_runner(self, batch: Batch):
+        """Runs whole blocks of this forward natively (``ops.block``); None where :meth:`_layer_forward` has to (CPU,
+        adapters, another layout or a subclass with its own block, forwards that record the QKV activations)."""
+        own = getattr(type(self), "_native_block_of", OPTModel)
         if (self.device.type != "cuda" or self.dtype != torch.bfloat16 or self.use_lora or self.use_prefix
                 or self.kv_capture is not None or gemm._VARIANT != 0
-                or type(self)._layer_forward is not OPTModel._layer_forward
-                or type(self)._layer_weights is not OPTModel._layer_weights
+                or type(self)._layer_forward is not own._layer_forward
+                or type(self)._layer_weights is not own._layer_weights
                 or type(self).hidden_states is not OPTModel.hidden_states):
             return None
+        return self._make_block_runner(batch)
+
+    def _make_block_runner(self, batch: Batch):
+        cfg = self.config
         B, L = batch.input_ids.shape
         return block_ops.BlockRunner(B, L, cfg.hidden_size, cfg.ffn_dim, cfg.num_attention_heads,
                                      cfg.do_layer_norm_before, gemm.ACT[cfg.activation_function], cfg.layer_norm_eps,
                                      batch.pad_left, self.device)
 
     def _block_weights(self, i: int, staged: torch.Tensor | None, shift: int, whole: bool) -> list[int] | None:
-        """Addresses of block ``i``'s weights in the order of ``ops.block.WEIGHTS``: in ``staged`` (a buffer laid out like
+        """Addresses of block ``i``'s weights in the order of ``_BLOCK_NAMES``: in ``staged`` (a buffer laid out like
         the arena from element ``shift`` on) the whole block, or with ``whole`` False its q | k | v weights only.  None
-        where q, k and v are not adjacent.  Only offsets are kept between calls."""
+        where the tensors of a fused operand are not adjacent.  Only offsets are kept between calls."""
         plan = self._block_plans.get(i)
         if plan is None:
-            lp = layer_prefix(i)
-            names = ["self_attn_layer_norm.weight", "self_attn_layer_norm.bias", "self_attn.q_proj.weight",
-                     "self_attn.q_proj.bias", "self_attn.out_proj.weight", "self_attn.out_proj.bias",
-                     "final_layer_norm.weight", "final_layer_norm.bias", "fc1.weight", "fc1.bias", "fc2.weight", "fc2.bias"]
-            plan = []
-            for n in names:
-                ar = self._where[lp + n]
-                plan.append((ar, ar.pieces[ar.index[lp + n]].offset, n.endswith("q_proj.weight")))
-            for wb in ("weight", "bias"):
-                ps = [self._where[f"{lp}self_attn.{x}_proj.{wb}"] for x in "qkv"]
-                pc = [ar.pieces[ar.index[f"{lp}self_attn.{x}_proj.{wb}"]] for ar, x in zip(ps, "qkv")]
-                if any(ar is not ps[0] for ar in ps) or any(b.offset != a.offset + a.numel for a, b in zip(pc, pc[1:])):
+            lp = self.layer_prefix(i)
+            where = lambda n: (self._where[lp + n], self._where[lp + n].pieces[self._where[lp + n].index[lp + n]])  # noqa: E731
+            plan = [(*where(n), n.endswith("q_proj.weight")) for n in self._BLOCK_NAMES]
+            plan = [(ar, p.offset, qkv) for ar, p, qkv in plan]
+            for group in self._BLOCK_FUSED:
+                ps = [where(n) for n in group]
+                if any(x[0] is not ps[0][0] or x[1].offset != y[1].offset + y[1].numel for y, x in zip(ps, ps[1:])):
                     plan = False
                     break
             self._block_plans[i] = plan

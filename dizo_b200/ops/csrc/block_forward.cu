@@ -1,4 +1,4 @@
-// A whole OPT decoder block launched by one call, and the choice of the GEMM kernel for a shape.
+// A whole OPT or LLaMA decoder block launched by one call, and the choice of the GEMM kernel for a shape.
 //
 // The seven kernels of a block run for 2 to 15 us each on the small models, but issued one by one from Python each costs
 // about 35 us of host time (tensor views, allocations, argument conversion).  A training step of OPT-125m, 16 prompts of 64
@@ -109,5 +109,77 @@ extern "C" int dz_opt_block(const DzOptBlock* blk, cudaStream_t stream) {
     if (!rc) rc = linear(b.f, b.fc2_w, b.fc2_b, b.h_mid, d, F, b.xn, 0);
     if (!rc) rc = norm(b.h_mid, b.ln2_w, b.ln2_b, b.h_out);
   }
+  return rc;
+}
+
+// Mirrored by ops/block.py.  A LLaMA-family block: RMSNorm, q | k | v with the rotary embedding, attention, output
+// projection, RMSNorm, SwiGLU, down projection.  The forms with the rotary embedding and SwiGLU in the GEMM's epilogue run
+// under the rules of ops/gemm.py (linear_qkv_rope, linear_swiglu); otherwise `raw` holds the plain projection in between.
+extern "C" struct DzLlamaBlock {
+  int B, L, d, F, H, Hkv, pos0, n_pos;
+  float eps, scale;
+  const void *ln1_w, *qkv_w, *out_w, *ln2_w, *gu_w, *down_w;
+  const void* h_in;                        // [B * L, d]
+  void *h_out, *h_mid, *xn, *qkv, *ctx, *f, *raw;   // raw: [B * L, max((H + 2 Hkv) hd, 2 F)], needed without the fused forms
+  const void* rope_cs;
+  const int* pad_left;
+  uint32_t* err;
+  int fused_rope, fused_swiglu;            // the options that switch the fused epilogues
+};
+
+extern "C" {
+int dz_rmsnorm(const void* x, long long ldx, const void* w, void* y, long long ldy, long long rows, int d, float eps,
+               cudaStream_t stream);
+int dz_rope_qkv(const void* in, long long ld_in, void* out, long long ld_out, const void* cs, long long rows, int L, int pos0,
+                int n_pos, int H, int Hkv, int hd, cudaStream_t stream);
+int dz_silu_mul(const void* gu, long long ld, void* out, long long ldo, long long rows, int F, cudaStream_t stream);
+int dz_gemm2_qkv_rope(const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo, const float* cs,
+                      int M, int K, int L, int pos0, int n_pos, int H, int Hkv, uint32_t* err, cudaStream_t stream);
+}
+
+static bool pairs_pay(int M, int N) { return M >= 256 && (long long)((M + 255) / 256) * (N / 256) >= 48; }
+
+// Bit 0: the projection with the rotary embedding is one kernel; bit 1: SwiGLU is.
+extern "C" int dz_llama_block_fused(int M, int H, int Hkv, int hd, int F, int fused_rope, int fused_swiglu) {
+  int r = 0;
+  if (fused_rope && hd == 128 && H % 2 == 0 && Hkv % 2 == 0 && pairs_pay(M, (H + 2 * Hkv) * hd)) r |= 1;
+  if (fused_swiglu && (M <= 64 || ((2 * F) % 256 == 0 && pairs_pay(M, 2 * F)))) r |= 2;
+  return r;
+}
+
+extern "C" int dz_llama_block(const DzLlamaBlock* blk, cudaStream_t stream) {
+  if (!blk || blk->B <= 0 || blk->L <= 0 || blk->H <= 0 || blk->Hkv <= 0 || blk->H % blk->Hkv || blk->d % blk->H ||
+      !blk->h_in || !blk->h_out || !blk->h_mid || !blk->xn || !blk->qkv || !blk->ctx || !blk->f || !blk->rope_cs)
+    return DZ_ERR_ARG;
+  const DzLlamaBlock& b = *blk;
+  if ((long long)b.B * b.L > 0x7fffffffLL) return DZ_ERR_TOO_LARGE;
+  const int M = b.B * b.L, d = b.d, F = b.F, hd = d / b.H, n_qkv = (b.H + 2 * b.Hkv) * hd;
+  const int fused = dz_llama_block_fused(M, b.H, b.Hkv, hd, F, b.fused_rope, b.fused_swiglu);
+  if (fused != 3 && !b.raw) return DZ_ERR_ARG;
+  auto linear = [&](const void* x, const void* w, void* y, int N, int K, const void* res) {
+    return dz_linear(x, K, w, K, y, N, nullptr, res, N, M, N, K, 0, 0, 1.0f, b.err, stream);
+  };
+  int rc = dz_rmsnorm(b.h_in, d, b.ln1_w, b.xn, d, M, d, b.eps, stream);
+  if (fused & 1) {
+    if (!rc) rc = dz_gemm2_qkv_rope(b.xn, d, b.qkv_w, d, b.qkv, 3 * d, static_cast<const float*>(b.rope_cs), M, d, b.L,
+                                    b.pos0, b.n_pos, b.H, b.Hkv, b.err, stream);
+  } else {
+    if (!rc) rc = linear(b.xn, b.qkv_w, b.raw, n_qkv, d, nullptr);
+    if (!rc) rc = dz_rope_qkv(b.raw, n_qkv, b.qkv, 3 * d, b.rope_cs, M, b.L, b.pos0, b.n_pos, b.H, b.Hkv, hd, stream);
+  }
+  if (!rc) rc = dz_attn_fwd(b.qkv, 3 * d, 0, d, 2 * d, b.ctx, d, b.pad_left, nullptr, nullptr, 0, 0, b.B, b.L, b.H, hd,
+                            b.scale, b.err, stream);
+  if (!rc) rc = linear(b.ctx, b.out_w, b.h_mid, d, d, b.h_in);
+  if (!rc) rc = dz_rmsnorm(b.h_mid, d, b.ln2_w, b.xn, d, M, d, b.eps, stream);
+  if (fused & 2) {
+    if (!rc && M <= 64)
+      rc = dz_gemm_skinny(b.xn, d, b.gu_w, d, b.f, F, nullptr, nullptr, 0, M, F, d, 3, 0, 1.0f, 0, b.err, stream);
+    else if (!rc)
+      rc = dz_gemm2_bf16_tn(b.xn, d, b.gu_w, d, b.f, F, nullptr, nullptr, 0, M, 2 * F, d, 3, 0, 1.0f, b.err, stream);
+  } else {
+    if (!rc) rc = linear(b.xn, b.gu_w, b.raw, 2 * F, d, nullptr);
+    if (!rc) rc = dz_silu_mul(b.raw, 2 * F, b.f, F, M, F, stream);
+  }
+  if (!rc) rc = linear(b.f, b.down_w, b.h_out, d, F, b.h_mid);
   return rc;
 }

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from dizo_b200.data.synthetic import synthetic_batch
+from dizo_b200.models.llama import LlamaConfig, LlamaModel
 from dizo_b200.models.opt import OPTConfig, OPTModel, Transform
 from dizo_b200.ops import _lib
 
@@ -38,6 +39,28 @@ def test_native_blocks_equal_layer_forward(pre, mode, d, B, L, monkeypatch):
         assert m._block_weights(0, None, 0, True) is not None
     native = results()
     monkeypatch.setattr(OPTModel, "_block_runner", lambda self, batch: None)
+    for x, y in zip(native, results()):
+        assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("heads,kv,d", [(4, 2, 512), (8, 8, 256)])          # head dims 128 and 32
+@pytest.mark.parametrize("mode", ["full", "head"])
+@pytest.mark.parametrize("B,L", [(1, 9), (3, 130), (16, 200)])
+def test_native_llama_blocks_equal_layer_forward(heads, kv, d, mode, B, L, monkeypatch):
+    cfg = LlamaConfig(vocab_size=520, hidden_size=d, num_hidden_layers=3, intermediate_size=712, num_attention_heads=heads,
+                      num_key_value_heads=kv, max_position_embeddings=256)
+    m = LlamaModel(cfg, "cuda", torch.bfloat16, mode=mode).init_random_fast(5, std=0.05)
+    b = synthetic_batch(1, B, L, 520, cand_ids=(9, 372)).to("cuda")
+    b.pad_left = torch.arange(B, dtype=torch.int32, device="cuda") % 5
+    assert m._block_runner(b) is not None and m._block_weights(0, None, 0, True) is not None
+
+    def results():
+        out = [m.hidden_states(b), m.hidden_states(b, Transform(seed=3, coef=1e-2), rows=b.rows), *m.loss_pair(b, 7, 1e-2)]
+        _lib.check_device_errors()
+        return out
+
+    native = results()
+    monkeypatch.setattr(LlamaModel, "_block_runner", lambda self, batch: None)
     for x, y in zip(native, results()):
         assert torch.equal(x, y)
 
