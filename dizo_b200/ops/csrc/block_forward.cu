@@ -7,6 +7,7 @@
 // The caller keeps one set of workspaces per forward and passes pointers; nothing is kept here between calls.
 #include "host_util.h"
 #include "linear.h"
+#include "skinny.h"
 
 extern "C" {
 int dz_layernorm(const void* x, long long ldx, const void* w, const void* b, void* y, long long ldy, long long rows, int d,
@@ -14,6 +15,9 @@ int dz_layernorm(const void* x, long long ldx, const void* w, const void* b, voi
 int dz_gemm_skinny(const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo, const void* bias,
                    const void* residual, long long ldr, int M, int N, int K, int act, int out_fp32, float out_scale,
                    int splits, uint32_t* err, cudaStream_t stream);
+int dz_gemv(const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo, const void* bias,
+            const void* residual, long long ldr, int M, int N, int K, int act, int out_fp32, float out_scale, uint32_t* err,
+            cudaStream_t stream);
 int dz_gemm2_bf16_tn(const void* A, long long lda, const void* W, long long ldw, void* out, long long ldo, const void* bias,
                      const void* residual, long long ldr, int M, int N, int K, int act, int out_fp32, float out_scale,
                      uint32_t* err, cudaStream_t stream);
@@ -54,6 +58,13 @@ extern "C" int dz_linear(const void* A, long long lda, const void* W, long long 
                          const void* bias, const void* residual, long long ldr, int M, int N, int K, int act,
                          int out_fp32, float out_scale, uint32_t* err, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return DZ_ERR_ARG;
+  // the vector kernel has no alignment rule for the output rows, the others do: what they refuse stays refused
+  const int esz = out_fp32 ? 4 : 2;
+  const bool rows_ok = !(reinterpret_cast<uintptr_t>(out) & 15) && !((ldo * esz) & 15) &&
+                       !(reinterpret_cast<uintptr_t>(bias) & 15) &&
+                       (!residual || (!(reinterpret_cast<uintptr_t>(residual) & 15) && !(ldr & 7)));
+  if (rows_ok && gemv_pays(M, N, K))
+    return dz_gemv(A, lda, W, ldw, out, ldo, bias, residual, ldr, M, N, K, act, out_fp32, out_scale, err, stream);
   const bool skinny = skinny_pays(M, N);
   const int splits = skinny || M <= 64 ? 0 : split_pays(M, N, K);
   if (skinny || splits)

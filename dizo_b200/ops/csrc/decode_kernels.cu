@@ -60,19 +60,23 @@ decode_attn_kernel(const DecodeAttnArgs p) {
     const int j = tid < half ? tid : tid - half;
     float2 cs = make_float2(1.f, 0.f);
     if (p.rope) cs = __ldg(p.rope + (long long)p.rope_pos * half + j);
+    // the new token's row is the predecessor's output: read past L1
+    auto fresh = [](const __nv_bfloat16* e) {
+      return __uint_as_float(static_cast<uint32_t>(__ldcg(reinterpret_cast<const unsigned short*>(e))) << 16);
+    };
     auto rotated = [&](const __nv_bfloat16* row) {
-      const float a = __bfloat162float(row[j]), c = __bfloat162float(row[j + half]);
+      const float a = fresh(row + j), c = fresh(row + j + half);
       const float r = tid < half ? a * cs.x - c * cs.y : c * cs.x + a * cs.y;
       return __bfloat162float(__float2bfloat16(r));           // q and k are held in bf16
     };
     const __nv_bfloat16* qr = p.q + (long long)b * p.ldq + h * hd;
-    s_q[tid] = (p.rope ? rotated(qr) : __bfloat162float(qr[tid])) * p.scale;
+    s_q[tid] = (p.rope ? rotated(qr) : fresh(qr + tid)) * p.scale;
     if (append) {
       const int hk = h / p.rep;
       const __nv_bfloat16* kr = p.k_new + (long long)b * p.ldq + hk * hd;
       const __nv_bfloat16* vr = p.v_new + (long long)b * p.ldq + hk * hd;
-      const float k = p.rope ? rotated(kr) : __bfloat162float(kr[tid]);
-      const float v = __bfloat162float(vr[tid]);
+      const float k = p.rope ? rotated(kr) : fresh(kr + tid);
+      const float v = fresh(vr + tid);
       s_kv[0][tid] = k;
       s_kv[1][tid] = v;
       if (rank == 0) {

@@ -8,7 +8,7 @@
 // way, so everything before the step (the weights included) is complete before any kernel of the step starts.
 //
 // Measured, per token: OPT-1.3b, one sequence of 300 tokens: 6.5 ms launched from Python, 1.44 ms from here without and
-// 1.10 ms with programmatic launches (the weights at the copy rate: 0.42 ms); LLaMA-2-7b, 16 sequences of 150: 3.80 and
+// 1.10 ms with programmatic launches, 0.99 with its products through gemv.cu (the weights at the copy rate: 0.42 ms); LLaMA-2-7b, 16 sequences of 150: 3.80 and
 // 3.34 ms (2.0 ms).  What is left is the chain of seven dependent kernels, about 3 us each beyond its bytes.
 #include <new>
 #include <vector>
@@ -47,6 +47,7 @@ struct LayerPlan {
 
 struct DecodePlan {
   DzDecodeConfig c;
+  bool vector;                         // gemv.cu for every product of a block
   CUtensorMap x_h, x_h2, x_xn, x_ctx, x_f;
   std::vector<LayerPlan> layers;
 };
@@ -74,9 +75,22 @@ int check(const DzDecodeConfig& c, const DzDecodeLayer* L) {
   return DZ_OK;
 }
 
+// Whether a block's products go through gemv.cu.  All or none: it lets its successor start only once its own input is there
+// (its reads need that), so a ring kernel behind it would lose its head start.  OPT-1.3b, one sequence, per token: 1.10 ms
+// through the ring kernel, 0.99 ms with all four products here, 1.09 with the two small ones.  Beyond about 20 Mi weights a
+// matrix, or with more rows beyond 6 Mi, the ring kernel reads W faster by more than the chain gains (gemv_pays).
+bool vector_pays(const DzDecodeConfig& c) {
+  const long long most = c.B == 1 ? 20LL << 20 : 6LL << 20;
+  const long long up = (long long)(c.act == 3 ? 2 : 1) * c.F * c.d;
+  const long long qkv = (long long)(c.H + 2 * c.Hkv) * c.hd * c.d;
+  return gemv_takes(c.B, c.d) && gemv_takes(c.B, c.F) && up <= most && qkv <= most && (long long)c.d * c.d <= most &&
+         (long long)c.d * c.F <= most;
+}
+
 int build(DecodePlan& p, const DzDecodeLayer* L) {
   const DzDecodeConfig& c = p.c;
   const int n_qkv = (c.H + 2 * c.Hkv) * c.hd;
+  p.vector = vector_pays(c);
   int rc = skinny_map_x(&p.x_h, c.h, c.d, c.B, c.d);
   if (!rc) rc = skinny_map_x(&p.x_h2, c.h2, c.d, c.B, c.d);
   if (!rc) rc = skinny_map_x(&p.x_xn, c.xn, c.d, c.B, c.d);
@@ -140,14 +154,15 @@ extern "C" int dz_decode_step(const void* plan, const void* const* k_cache, cons
     return c.rms ? rmsnorm_launch(B16(x), c.d, B16(w), o, c.d, c.B, c.d, c.eps, dep, stream)
                  : layernorm_launch(B16(x), c.d, B16(w), B16(b), o, c.d, c.B, c.d, c.eps, dep, stream);
   };
-  auto gemm = [&](const CUtensorMap& w, const CUtensorMap& x, void* out, int N, int K, const void* bias,
-                  const void* residual, int act) {
+  auto gemm = [&](const CUtensorMap& w, const CUtensorMap& x, const void* W, const void* X, void* out, int N, int K,
+                  const void* bias, const void* residual, int act) {
     SkinnyArgs a{};
     a.M = c.B; a.N = N; a.K = K; a.out = out; a.ldo = N; a.bias = B16(bias); a.residual = B16(residual);
     a.ldr = N; a.act = act; a.out_scale = 1.0f; a.err = c.err;
     a.w_static = first ? 0 : 1;
     const bool dep = !first;
     first = false;
+    if (p.vector) return gemv_launch(W, K, X, K, a, dep, stream);
     return skinny_launch(w, x, a, 0, dep, stream);
   };
   for (int i = 0; i < c.layers; ++i) {
@@ -155,7 +170,7 @@ extern "C" int dz_decode_step(const void* plan, const void* const* k_cache, cons
     if (!k_cache[i] || !v_cache[i]) return DZ_ERR_ARG;
     int rc = DZ_OK;
     if (c.pre_norm) rc = norm(c.h, l.w.ln1_w, l.w.ln1_b, c.xn);
-    if (!rc) rc = gemm(l.qkv, c.pre_norm ? p.x_xn : p.x_h, c.qkv, n_qkv, c.d, l.w.qkv_b, nullptr, 0);
+    if (!rc) rc = gemm(l.qkv, c.pre_norm ? p.x_xn : p.x_h, l.w.qkv_w, c.pre_norm ? c.xn : c.h, c.qkv, n_qkv, c.d, l.w.qkv_b, nullptr, 0);
     if (rc) return rc;
     DecodeAttnArgs a{};
     a.q = B16(c.qkv); a.ldq = n_qkv;
@@ -173,15 +188,15 @@ extern "C" int dz_decode_step(const void* plan, const void* const* k_cache, cons
     rc = decode_attn_launch(a, c.B, c.H, true, stream);
     if (rc) return rc;
     if (c.pre_norm) {
-      rc = gemm(l.out, p.x_ctx, c.h, c.d, c.d, l.w.out_b, c.h, 0);
+      rc = gemm(l.out, p.x_ctx, l.w.out_w, c.ctx, c.h, c.d, c.d, l.w.out_b, c.h, 0);
       if (!rc) rc = norm(c.h, l.w.ln2_w, l.w.ln2_b, c.xn);
-      if (!rc) rc = gemm(l.up, p.x_xn, c.f, c.F, c.d, l.w.up_b, nullptr, c.act);
-      if (!rc) rc = gemm(l.down, p.x_f, c.h, c.d, c.F, l.w.down_b, c.h, 0);
+      if (!rc) rc = gemm(l.up, p.x_xn, l.w.up_w, c.xn, c.f, c.F, c.d, l.w.up_b, nullptr, c.act);
+      if (!rc) rc = gemm(l.down, p.x_f, l.w.down_w, c.f, c.h, c.d, c.F, l.w.down_b, c.h, 0);
     } else {
-      rc = gemm(l.out, p.x_ctx, c.h2, c.d, c.d, l.w.out_b, c.h, 0);
+      rc = gemm(l.out, p.x_ctx, l.w.out_w, c.ctx, c.h2, c.d, c.d, l.w.out_b, c.h, 0);
       if (!rc) rc = norm(c.h2, l.w.ln1_w, l.w.ln1_b, c.h);
-      if (!rc) rc = gemm(l.up, p.x_h, c.f, c.F, c.d, l.w.up_b, nullptr, c.act);
-      if (!rc) rc = gemm(l.down, p.x_f, c.h2, c.d, c.F, l.w.down_b, c.h, 0);
+      if (!rc) rc = gemm(l.up, p.x_h, l.w.up_w, c.h, c.f, c.F, c.d, l.w.up_b, nullptr, c.act);
+      if (!rc) rc = gemm(l.down, p.x_f, l.w.down_w, c.f, c.h2, c.d, c.F, l.w.down_b, c.h, 0);
       if (!rc) rc = norm(c.h2, l.w.ln2_w, l.w.ln2_b, c.h);
     }
     if (rc) return rc;

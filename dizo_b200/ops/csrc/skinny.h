@@ -32,4 +32,10 @@ int skinny_map_x(CUtensorMap* map, const void* A, long long lda, int M, int K);
 int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, int splits, bool dependent,
                   cudaStream_t stream);
 
+// One to four rows without tensor cores (gemv.cu), where gemv_takes(); worth it where gemv_pays().
+bool gemv_takes(int M, int K);
+bool gemv_pays(int M, int N, int K);
+int gemv_launch(const void* W, long long ldw, const void* A, long long lda, const SkinnyArgs& a, bool dependent,
+                cudaStream_t stream);
+
 }  // namespace dz

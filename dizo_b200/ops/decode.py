@@ -105,6 +105,7 @@ class DecodePlan:
         ws = lambda n: torch.empty((B, n), dtype=torch.bfloat16, device=dev)          # noqa: E731
         self.h, self._ws = ws(d), [ws(d), ws(d), ws((H + 2 * Hkv) * hd), ws(d), ws(F)]
         self._keep = (layers, rope)
+        self._kernels = 7 * len(layers)
         pk = layers[0].get("prefix_k")
         for w in layers:
             for n in _LAYER_FIELDS:
@@ -129,6 +130,7 @@ class DecodePlan:
         rc = _lib.lib().dz_decode_step(self._handle, caches[0], caches[1], int(t), _lib.ptr(pad_left),
                                        _lib.stream_ptr())
         _lib.check(rc, "dz_decode_step")
+        _lib.launch_count += self._kernels - 1               # check() counted one
         return self.h
 
     def __del__(self):

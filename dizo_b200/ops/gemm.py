@@ -116,6 +116,16 @@ def _skinny(x2, w, out2, bias, res2, act: int, scale: float, splits: int = 0) ->
     _lib.check(rc, "dz_gemm_skinny")
 
 
+def _gemv(x2, w, out2, bias, res2, act: int, scale: float) -> None:
+    """``out2 = epilogue(x2 @ w.T)`` for one to four rows (``act`` as in :func:`_skinny`)."""
+    rc = _lib.lib().dz_gemv(
+        _lib.ptr(x2), ctypes.c_longlong(x2.stride(0)), _lib.ptr(w), ctypes.c_longlong(w.stride(0)),
+        _lib.ptr(out2), ctypes.c_longlong(out2.stride(0)), _lib.ptr(bias), _lib.ptr(res2),
+        ctypes.c_longlong(res2.stride(0) if res2 is not None else 0), x2.shape[0], out2.shape[1], x2.shape[1], act,
+        int(out2.dtype == torch.float32), ctypes.c_float(scale), _lib.ptr(_lib.err_word(x2.device)), _lib.stream_ptr())
+    _lib.check(rc, "dz_gemv")
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, act: str | None = None,
            residual: torch.Tensor | None = None, scale: float = 1.0,
            out_dtype: torch.dtype | None = None, out: torch.Tensor | None = None,

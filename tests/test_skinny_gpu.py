@@ -49,3 +49,24 @@ def test_skinny_swiglu(M, F, K):
     ref = torch.nn.functional.silu(gu[:, :F]) * gu[:, F:]
     # __expf and the fast division are good to a few fp32 ulp: far below the bf16 rounding of the result
     _close(y, ref, K)
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("N,K", [(1, 8), (8, 2048), (201, 2056), (1032, 8200), (2048, 11008), (25001, 136)])
+def test_gemv(M, N, K):
+    x, w, r, b = _rand(M, K, seed=1), _rand(N, K, seed=2, scale=0.05), _rand(M, N, seed=3), _rand(N, seed=4)
+    for dtype, act in ((torch.bfloat16, "relu"), (torch.float32, None)):
+        out = torch.full((M, N), float("nan"), dtype=dtype, device="cuda")
+        gemm._gemv(x, w, out, b, r, gemm.ACT[act], 0.5)
+        _close(out, gemm.linear_reference(x, w, b, act=act, residual=r, scale=0.5, out_dtype=torch.float32), K)
+    if N % 2 == 0:
+        out = torch.empty((M, N // 2), dtype=torch.bfloat16, device="cuda")
+        gemm._gemv(x, w, out, None, None, 3, 1.0)
+        gu = x.float() @ w.float().t()
+        _close(out, torch.nn.functional.silu(gu[:, :N // 2]) * gu[:, N // 2:], K)
+
+
+def test_gemv_limits():
+    x, w = _rand(4, 20480, seed=1), _rand(64, 20480, seed=2)
+    with pytest.raises(_lib.KernelError):
+        gemm._gemv(x, w, torch.empty((4, 64), dtype=torch.bfloat16, device="cuda"), None, None, 0, 1.0)
