@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from dizo_b200.models.generate import _Decoder
+from dizo_b200.models.generate import _Decoder, generate
 from dizo_b200.models.llama import LlamaConfig, LlamaModel
 from dizo_b200.models.opt import OPTConfig, OPTModel, make_batch
 from dizo_b200.ops import _lib
@@ -89,3 +89,21 @@ def test_sample_step_marks_finished_rows():
     eos = torch.tensor([4, 60], dtype=torch.int32, device="cuda")
     out = decode_ops.sample_step(logits, do_sample=False, done=done, eos=eos, pad_id=1)
     assert out.tolist() == [9, 4, 1] and done.tolist() == [0, 1, 1]
+
+
+@pytest.mark.parametrize("sample", [False, True])
+def test_generate_stops_rows_at_an_end_of_sequence_id(sample):
+    """The step that is queued before the host sees a token changes nothing: rows end with their first EOS id."""
+    m = _models()["opt"]().init_random_fast(3, std=0.05)
+    g = torch.Generator().manual_seed(4)
+    ids = torch.randint(4, 500, (3, 20), generator=g)
+    mask = torch.ones_like(ids)
+    mask[1, :7] = 0
+    kw = dict(max_new_tokens=9, do_sample=sample, top_p=0.9, seed=3)
+    free = generate(m, ids, mask, **kw)
+    for stop in ({free[0][21]}, {row[-3] for row in free}):
+        got = generate(m, ids, mask, eos_token_id=sorted(stop), pad_token_id=1, **kw)
+        for row, prompt, out in zip(free, (20, 13, 20), got):
+            end = next((i + 1 for i in range(prompt, len(row)) if row[i] in stop), len(row))
+            assert out == row[:end]
+    assert generate(m, ids, mask, max_new_tokens=0) == [r[k.bool()].tolist() for r, k in zip(ids, mask)]
