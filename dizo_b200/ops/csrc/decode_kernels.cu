@@ -59,7 +59,7 @@ decode_attn_kernel(const DecodeAttnArgs p) {
     const int half = hd >> 1;
     const int j = tid < half ? tid : tid - half;
     float2 cs = make_float2(1.f, 0.f);
-    if (p.rope) cs = __ldg(p.rope + (long long)p.rope_pos * half + j);
+    if (p.rope) cs = ld_table(p.rope + (long long)p.rope_pos * half + j);
     // the new token's row is the predecessor's output: read past L1
     auto fresh = [](const __nv_bfloat16* e) {
       return __uint_as_float(static_cast<uint32_t>(__ldcg(reinterpret_cast<const unsigned short*>(e))) << 16);

@@ -254,7 +254,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             if (is_q || is_k) {
 #pragma unroll
               for (int i = 0; i < 16; ++i) {
-                const float4 c = __ldg(csr + pc * 16 + i);       // (cos, sin) of frequencies 2i and 2i + 1
+                const float4 c = ld_table(csr + pc * 16 + i);       // (cos, sin) of frequencies 2i and 2i + 1
                 const float a0 = __uint_as_float(a[2 * i]), a1 = __uint_as_float(a[2 * i + 1]);
                 const float b0 = __uint_as_float(b[2 * i]), b1 = __uint_as_float(b[2 * i + 1]);
                 lo[2 * i] = a0 * c.x - b0 * c.y;      lo[2 * i + 1] = a1 * c.z - b1 * c.w;
@@ -345,7 +345,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             const uint4* bp = reinterpret_cast<const uint4*>(p.bias + col0);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              uint4 b = __ldg(bp + q);
+              const uint4 b = __ldca(bp + q);
               v[q * 8 + 0] += bf16_lo(b.x); v[q * 8 + 1] += bf16_hi(b.x);
               v[q * 8 + 2] += bf16_lo(b.y); v[q * 8 + 3] += bf16_hi(b.y);
               v[q * 8 + 4] += bf16_lo(b.z); v[q * 8 + 5] += bf16_hi(b.z);

@@ -237,7 +237,7 @@ gemm_bf16_tn_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
               const uint4* bp = reinterpret_cast<const uint4*>(p.bias + col0);
 #pragma unroll
               for (int q = 0; q < 4; ++q) {
-                uint4 b = __ldg(bp + q);
+                const uint4 b = __ldca(bp + q);
                 v[q * 8 + 0] += bf16_lo(b.x); v[q * 8 + 1] += bf16_hi(b.x);
                 v[q * 8 + 2] += bf16_lo(b.y); v[q * 8 + 3] += bf16_hi(b.y);
                 v[q * 8 + 4] += bf16_lo(b.z); v[q * 8 + 5] += bf16_hi(b.z);

@@ -19,9 +19,10 @@ constexpr int GV_K = GV_CHUNKS * 32 * 8;         // columns of W per warp
 constexpr int GV_WARPS = 10;                     // most warps of a CTA (K up to 20480)
 constexpr int GV_SMEM = 96 * 1024;               // A of a CTA
 
+// Coherent: outside a decoding step the sweep that stages W may have been launched just ahead (pdl.cuh).
 __device__ __forceinline__ uint4 ld_weight(const __nv_bfloat16* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
@@ -29,7 +30,7 @@ __device__ __forceinline__ uint4 ld_weight(const __nv_bfloat16* p) {
 // ks: warps that share a row pair; groups: row pairs per CTA.
 template <int M>
 __global__ void __launch_bounds__(GV_WARPS * 32)
-gemv_kernel(const __nv_bfloat16* __restrict__ W, long long ldw, const __nv_bfloat16* A, long long lda, const SkinnyArgs p,
+gemv_kernel(const __nv_bfloat16* W, long long ldw, const __nv_bfloat16* A, long long lda, const SkinnyArgs p,
             int ks, int groups) {
   extern __shared__ __align__(16) uint8_t gv_smem[];          // A as [M][K] bf16
   __shared__ float s_part[GV_WARPS][2 * M];

@@ -21,7 +21,7 @@ constexpr int RMS_MAXV = 4;  // uint4 (8 bf16) per thread held in registers
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
-rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bfloat16* __restrict__ w,
+rmsnorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w,
                __nv_bfloat16* __restrict__ y, long long ldy, int d, float eps) {
   __shared__ float s_red[THREADS / 32];
   pdl_trigger();
@@ -52,16 +52,23 @@ rmsnorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const __nv_bf
   const float rstd = rsqrtf(tot / d + eps);
   uint4* yr = reinterpret_cast<uint4*>(y + row * ldy);
   const uint4* wr = reinterpret_cast<const uint4*>(w);
+  // coherent loads: the sweep right in front of this kernel may have written w (pdl.cuh).  All before the first store,
+  // which they may not pass.
+  uint4 wv[RMS_MAXV];
+#pragma unroll
+  for (int i = 0; i < RMS_MAXV; ++i) {
+    const int idx = threadIdx.x + i * THREADS;
+    if (idx < nvec) wv[i] = __ldca(wr + idx);
+  }
 #pragma unroll
   for (int i = 0; i < RMS_MAXV; ++i) {
     const int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
-      const uint4 wv = __ldg(wr + idx);
       uint4 o;
-      o.x = pack_bf16x2(bf16_lo(v[i].x) * rstd * bf16_lo(wv.x), bf16_hi(v[i].x) * rstd * bf16_hi(wv.x));
-      o.y = pack_bf16x2(bf16_lo(v[i].y) * rstd * bf16_lo(wv.y), bf16_hi(v[i].y) * rstd * bf16_hi(wv.y));
-      o.z = pack_bf16x2(bf16_lo(v[i].z) * rstd * bf16_lo(wv.z), bf16_hi(v[i].z) * rstd * bf16_hi(wv.z));
-      o.w = pack_bf16x2(bf16_lo(v[i].w) * rstd * bf16_lo(wv.w), bf16_hi(v[i].w) * rstd * bf16_hi(wv.w));
+      o.x = pack_bf16x2(bf16_lo(v[i].x) * rstd * bf16_lo(wv[i].x), bf16_hi(v[i].x) * rstd * bf16_hi(wv[i].x));
+      o.y = pack_bf16x2(bf16_lo(v[i].y) * rstd * bf16_lo(wv[i].y), bf16_hi(v[i].y) * rstd * bf16_hi(wv[i].y));
+      o.z = pack_bf16x2(bf16_lo(v[i].z) * rstd * bf16_lo(wv[i].z), bf16_hi(v[i].z) * rstd * bf16_hi(wv[i].z));
+      o.w = pack_bf16x2(bf16_lo(v[i].w) * rstd * bf16_lo(wv[i].w), bf16_hi(v[i].w) * rstd * bf16_hi(wv[i].w));
       if (DZ_STORE_OK(yr + idx, 16)) yr[idx] = o;
     }
   }

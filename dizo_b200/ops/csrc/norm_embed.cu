@@ -19,8 +19,7 @@ constexpr int LN_MAXV = 4;  // uint4 (8 bf16) per thread held in registers
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
-layernorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
-                 const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
+layernorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* b,
                  __nv_bfloat16* __restrict__ y, long long ldy, int d, float eps) {
   __shared__ float s_red[THREADS / 32];
   __shared__ float s_bcast;
@@ -74,20 +73,30 @@ layernorm_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
   uint4* yr = reinterpret_cast<uint4*>(y + row * ldy);
   const uint4* wr = reinterpret_cast<const uint4*>(w);
   const uint4* br = reinterpret_cast<const uint4*>(b);
+  // coherent loads: the sweep right in front of this kernel may have written w and b (pdl.cuh).  All before the first
+  // store, which they may not pass.
+  uint4 wv[LN_MAXV], bv[LN_MAXV];
+#pragma unroll
+  for (int i = 0; i < LN_MAXV; ++i) {
+    const int idx = threadIdx.x + i * THREADS;
+    if (idx < nvec) {
+      wv[i] = __ldca(wr + idx);
+      bv[i] = __ldca(br + idx);
+    }
+  }
 #pragma unroll
   for (int i = 0; i < LN_MAXV; ++i) {
     int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
-      uint4 wv = __ldg(wr + idx), bv = __ldg(br + idx);
       uint4 o;
-      o.x = pack_bf16x2((bf16_lo(v[i].x) - mean) * rstd * bf16_lo(wv.x) + bf16_lo(bv.x),
-                        (bf16_hi(v[i].x) - mean) * rstd * bf16_hi(wv.x) + bf16_hi(bv.x));
-      o.y = pack_bf16x2((bf16_lo(v[i].y) - mean) * rstd * bf16_lo(wv.y) + bf16_lo(bv.y),
-                        (bf16_hi(v[i].y) - mean) * rstd * bf16_hi(wv.y) + bf16_hi(bv.y));
-      o.z = pack_bf16x2((bf16_lo(v[i].z) - mean) * rstd * bf16_lo(wv.z) + bf16_lo(bv.z),
-                        (bf16_hi(v[i].z) - mean) * rstd * bf16_hi(wv.z) + bf16_hi(bv.z));
-      o.w = pack_bf16x2((bf16_lo(v[i].w) - mean) * rstd * bf16_lo(wv.w) + bf16_lo(bv.w),
-                        (bf16_hi(v[i].w) - mean) * rstd * bf16_hi(wv.w) + bf16_hi(bv.w));
+      o.x = pack_bf16x2((bf16_lo(v[i].x) - mean) * rstd * bf16_lo(wv[i].x) + bf16_lo(bv[i].x),
+                        (bf16_hi(v[i].x) - mean) * rstd * bf16_hi(wv[i].x) + bf16_hi(bv[i].x));
+      o.y = pack_bf16x2((bf16_lo(v[i].y) - mean) * rstd * bf16_lo(wv[i].y) + bf16_lo(bv[i].y),
+                        (bf16_hi(v[i].y) - mean) * rstd * bf16_hi(wv[i].y) + bf16_hi(bv[i].y));
+      o.z = pack_bf16x2((bf16_lo(v[i].z) - mean) * rstd * bf16_lo(wv[i].z) + bf16_lo(bv[i].z),
+                        (bf16_hi(v[i].z) - mean) * rstd * bf16_hi(wv[i].z) + bf16_hi(bv[i].z));
+      o.w = pack_bf16x2((bf16_lo(v[i].w) - mean) * rstd * bf16_lo(wv[i].w) + bf16_lo(bv[i].w),
+                        (bf16_hi(v[i].w) - mean) * rstd * bf16_hi(wv[i].w) + bf16_hi(bv[i].w));
       if (DZ_STORE_OK(yr + idx, 16)) yr[idx] = o;
     }
   }

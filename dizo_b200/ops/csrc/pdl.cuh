@@ -4,8 +4,11 @@
 // predecessor has completed and its memory is visible, and because every kernel of such a chain waits before it
 // finishes, so has everything launched before it.  Both instructions do nothing in a kernel launched the ordinary way.
 //
-// Between its start and pdl_wait() a kernel shares the chip with its predecessors, so what they produce is never read with
-// non-coherent loads (ld.global.nc, __ldg): those are for weights and tables, complete many launches earlier.
+// A whole chain of such kernels can be resident while its first one still writes (each triggers before it waits): the norm
+// behind a staging sweep, the projection behind the norm and so on, with the weights of all of them in the sweep's output.
+// Memory that is written during a kernel's lifetime may not be read with non-coherent loads, so a kernel that calls
+// pdl_wait() has no ld.global.nc, no __ldg and no `const __restrict__` parameter (through which the compiler may issue
+// either), for weights and biases no more than for activations.  The exception is ld_table(): constants that nothing rewrites.
 //
 // The GEMMs, the attention forward, the norms and the sweeps always launch this way (a kernel launched the ordinary way in
 // between serialises as before): the launch latency and the set-up of barriers, TMEM and tables run beside the predecessor's
@@ -21,6 +24,10 @@ namespace dz {
 
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A constant that no kernel of the process rewrites (quantiles, rotary angles).
+template <class T>
+__device__ __forceinline__ T ld_table(const T* p) { return __ldg(p); }
 
 // Launch with an optional cluster of `cluster_x` CTAs along x, optionally as a programmatic dependent.
 template <class... Params, class... Args>

@@ -238,7 +238,7 @@ zo_sweep_kernel(const ZoSweepArgs a_in) {
   const char* tab;
   if (SMALL) {
     for (int i = threadIdx.x; i < GAUSS_BINS; i += THREADS)
-      reinterpret_cast<uint32_t*>(zo_smem)[i] = __ldg(a.gauss_table + i);
+      reinterpret_cast<uint32_t*>(zo_smem)[i] = ld_table(a.gauss_table + i);
     tab = reinterpret_cast<const char*>(zo_smem);
   } else {
     gauss_table_to_smem(zo_smem, a.gauss_table, threadIdx.x, THREADS);

@@ -76,3 +76,39 @@ def test_native_block_does_not_overwrite_its_input():
     assert torch.equal(h, keep)
     z = r.run(h, ptrs, out=h)
     assert z.data_ptr() == h.data_ptr() and torch.equal(z, y)
+
+
+@pytest.mark.parametrize("family", ["opt", "opt-post", "llama"])
+@pytest.mark.parametrize("B,L", [(1, 9), (3, 40)])           # the last block's tail has 1 and 3 rows: register products
+def test_staged_weights_in_a_chain_equal_a_synchronised_one(family, B, L, monkeypatch):
+    """Every block reads weights that the sweep in front of it has just written into a reused buffer.  A chain of dependent
+    launches gives the bits of the same kernels with the device idle before each of them."""
+    if family == "llama":
+        m = LlamaModel(LlamaConfig(vocab_size=520, hidden_size=256, num_hidden_layers=6, intermediate_size=712,
+                                   num_attention_heads=4, num_key_value_heads=2, max_position_embeddings=256), "cuda",
+                       torch.bfloat16).init_random_fast(5, std=0.05)
+    else:
+        m = OPTModel(OPTConfig(vocab_size=520, hidden_size=256, num_hidden_layers=6, ffn_dim=520, num_attention_heads=4,
+                               max_position_embeddings=160, do_layer_norm_before=family == "opt",
+                               word_embed_proj_dim=256 if family == "opt" else 64), "cuda",
+                     torch.bfloat16).init_random_fast(5, std=0.05)
+    b = synthetic_batch(1, B, L, 520, cand_ids=(9, 372)).to("cuda")
+
+    def results():
+        out = []
+        for seed in range(4):
+            out += [*m.loss_pair(b, seed, 0.3), m.hidden_states(b, Transform(seed=seed, coef=0.3), rows=b.rows)]
+        _lib.check_device_errors()
+        return out
+
+    chained = results()
+    check = _lib.check
+
+    def waiting(rc, name):
+        torch.cuda.synchronize()
+        check(rc, name)
+
+    monkeypatch.setattr(_lib, "check", waiting)
+    monkeypatch.setattr(type(m), "_block_runner", lambda self, batch: None)       # one Python call a kernel
+    for x, y in zip(chained, results()):
+        assert torch.equal(x, y)
