@@ -114,6 +114,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     if (elect_one()) {
       // ---------------------------------------------------------- MMA issuer
       constexpr uint32_t idesc = umma_idesc_bf16(SK_BM, NB);
+      pdl_wait();                     // the time limits below count from here, not from an early start beside predecessors
       bool ok = true;
       for (int i = 0; i < n_kb; ++i) {
         const int stage = i % S::STAGES;
@@ -132,6 +133,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   } else {
     // ------------------------------------------------------------ accumulator -> partial tile [row][feature]
     const int quad = warp & 3;
+    pdl_wait();                       // as above; and the residual below is the predecessor's output, `out` may be its input
     if (mbar_wait(smem_u32(&bar_acc), 0, &s_abort, p.err, ERR_WAIT_TMEM_FULL)) {
       // every stage has been read by a finished MMA: the ring is free to hold the partial tile
       tc_fence_after();
@@ -147,7 +149,6 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + (c + j) * (SK_BM * 4)), "r"(r[j]) : "memory");
       }
     }
-    pdl_wait();                       // the residual below is the predecessor's output, and `out` may be its input
   }
   __syncwarp();
   tc_fence_before();
