@@ -58,9 +58,10 @@ class _Decoder:
         cfg = model.config
         d = cfg.hidden_size
         dev, dt = model.device, model.dtype
-        # columns are written before they are read: no initial value
-        kv = torch.empty(2 * cfg.num_hidden_layers, B, max_len, d, dtype=dt, device=dev)
-        self.k, self.v = list(kv[0::2]), list(kv[1::2])
+        # one allocation a tensor: reordering beams replaces them one by one, and each one's memory goes back as it is
+        # replaced.  Columns are written before they are read: no initial value.
+        self.k = [torch.empty(B, max_len, d, dtype=dt, device=dev) for _ in range(cfg.num_hidden_layers)]
+        self.v = [torch.empty(B, max_len, d, dtype=dt, device=dev) for _ in range(cfg.num_hidden_layers)]
         self.len = 0
         self.plan, self._caches = None, None
         self.native = (dev.type == "cuda" and dt == torch.bfloat16 and B <= decode_ops.MAX_STEP_ROWS

@@ -1,0 +1,18 @@
+"""Host side of decoding: the caches of a run."""
+import torch
+
+from dizo_b200.models.generate import _Decoder
+from dizo_b200.models.opt import OPTConfig, OPTModel
+
+
+def test_each_cache_owns_its_memory():
+    """Reordering beams replaces the caches one by one: what is replaced can go back at once only if no other cache is a
+    view of the same allocation."""
+    m = OPTModel(OPTConfig(vocab_size=60, hidden_size=32, num_hidden_layers=3, ffn_dim=64, num_attention_heads=2,
+                           max_position_embeddings=64), "cpu", torch.float32)
+    dec = _Decoder(m, 4, 10)
+    for _ in range(2):
+        tensors = dec.k + dec.v
+        assert len({t.untyped_storage().data_ptr() for t in tensors}) == len(tensors) == 6
+        assert all(t.untyped_storage().nbytes() == 4 * 10 * 32 * 4 for t in tensors)
+        dec.reorder(torch.tensor([1, 0, 3, 3]))
