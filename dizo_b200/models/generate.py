@@ -79,8 +79,7 @@ class _Decoder:
             self.native = False
             return
         B, max_len, d = self.k[0].shape
-        self.plan = decode_ops.DecodePlan(layers, B=B, d=d, ld_seq=max_len * d, ld_row=d,
-                                          **m.step_config(m.num_prefix + max_len))
+        self.plan = decode_ops.DecodePlan(layers, B=B, d=d, cache_rows=max_len, **m.step_config(m.num_prefix + max_len))
 
     def prefill(self, batch: Batch) -> torch.Tensor:
         m = self.m
@@ -118,8 +117,9 @@ class _Decoder:
             if self._caches is None:
                 self._caches = self.plan.caches(self.k, self.v)
             self.plan.h.copy_(h)
+            h = self.plan.step(self._caches, t, pad_left)
             self.len = t + 1
-            return _head_logits(m, self.plan.step(self._caches, t, pad_left))
+            return _head_logits(m, h)
         for i in range(m.config.num_hidden_layers):
             w = m._layer_weights(i, m._resolver(i, None, None, 0))
             h = m.decode_block(h, w, self.k[i], self.v[i], t, pad_left)

@@ -5,6 +5,10 @@
 
 namespace dz {
 
+// Keys of one (sequence, head), prefix rows among them.  The kernel itself keeps no scores; the bound on the length of a
+// sequence is what the entry points refuse.
+constexpr int DA_MAX_KEYS = 40 * 1024;
+
 struct DecodeAttnArgs {
   const __nv_bfloat16* q;              // [B, ldq], head h at column h * hd
   long long ldq;

@@ -81,8 +81,8 @@ decode_attn_kernel(const DecodeAttnArgs p) {
       s_kv[1][tid] = v;
       if (rank == 0) {
         const long long at = seq + (long long)cached * p.ld_row + tid;
-        p.kc[at] = __float2bfloat16(k);
-        p.vc[at] = __float2bfloat16(v);
+        if (DZ_STORE_OK(p.kc + at, 2)) p.kc[at] = __float2bfloat16(k);
+        if (DZ_STORE_OK(p.vc + at, 2)) p.vc[at] = __float2bfloat16(v);
       }
     }
   }
@@ -190,7 +190,8 @@ decode_attn_kernel(const DecodeAttnArgs p) {
       ll = fmaf(s_l[w], f, ll);
     }
     if (p.splits == 1) {
-      p.out[(long long)b * p.ldo + h * hd + tid] = __float2bfloat16(o / ll);
+      __nv_bfloat16* op = p.out + (long long)b * p.ldo + h * hd + tid;
+      if (DZ_STORE_OK(op, 2)) *op = __float2bfloat16(o / ll);
     } else {
       s_cta[2 + tid] = o;
       if (tid == 0) { s_cta[0] = mm; s_cta[1] = ll; }
@@ -218,7 +219,8 @@ decode_attn_kernel(const DecodeAttnArgs p) {
         o = fmaf(os[r], f, o);
         ll = fmaf(ls[r], f, ll);
       }
-      p.out[(long long)b * p.ldo + h * hd + tid] = __float2bfloat16(o / ll);
+      __nv_bfloat16* op = p.out + (long long)b * p.ldo + h * hd + tid;
+      if (DZ_STORE_OK(op, 2)) *op = __float2bfloat16(o / ll);
     }
     __syncwarp();
     cluster_sync_all();                       // nobody leaves while rank 0 may still read its partial result
@@ -289,10 +291,10 @@ sample_topk_topp_kernel(const float* __restrict__ logits, long long ld, int V, f
         tok = pad_id;
       } else {
         for (int e = 0; e < n_eos; ++e)
-          if (tok == eos[e]) done[row] = 1;
+          if (tok == eos[e] && DZ_STORE_OK(done + row, 4)) done[row] = 1;
       }
     }
-    out[row] = tok;
+    if (DZ_STORE_OK(out + row, 4)) out[row] = tok;
   };
   const float inv_t = (do_sample && temperature > 0.f) ? 1.0f / temperature : 1.0f;
   // ---- maximum (and argmax with the lowest index on ties)
@@ -443,6 +445,7 @@ sample_topk_topp_kernel(const float* __restrict__ logits, long long ld, int V, f
 }  // namespace dz
 
 using namespace dz;
+DZ_DEBUG_TU(decode)
 
 extern "C" int dz_decode_attn(const void* q, long long ldq, const void* kc, const void* vc,
                               long long ld_seq, long long ld_row, const void* pk, const void* pv,
@@ -452,7 +455,7 @@ extern "C" int dz_decode_attn(const void* q, long long ldq, const void* kc, cons
   if (!q || !kc || !vc || !out || B <= 0 || H <= 0 || kv_len <= 0) return DZ_ERR_ARG;
   if (hd > 128 || (hd & 7) || (ld_row & 7) || (ld_seq & 7) || (n_prefix > 0 && (!pk || !pv || (ldp & 7))))
     return DZ_ERR_ARG;
-  if (sizeof(float) * (size_t)(n_prefix + kv_len) > 160 * 1024) return DZ_ERR_TOO_LARGE;
+  if ((long long)n_prefix + kv_len > DA_MAX_KEYS) return DZ_ERR_TOO_LARGE;
   DecodeAttnArgs a{};
   a.q = (const __nv_bfloat16*)q; a.ldq = ldq;
   // without a new key the cache is only read

@@ -29,6 +29,7 @@ extern "C" struct DzDecodeConfig {
   int pre_norm;        // norms in front of the sub-layers (else behind the residual sums)
   int act;             // of the FFN: 1 relu, 2 gelu, 3 SwiGLU (up_w = gate rows | up rows)
   int rope_n_pos;      // 0: no rotary embedding
+  int cache_rows;      // rows of a sequence in the caches: a step at or past it is refused
   float eps, scale;
   long long ld_prefix, ld_seq, ld_row;
   const void* rope_cs; // fp32 [rope_n_pos][hd / 2][2]
@@ -57,7 +58,7 @@ bool al16_or_null(const void* p) { return !(reinterpret_cast<uintptr_t>(p) & 15)
 
 int check(const DzDecodeConfig& c, const DzDecodeLayer* L) {
   if (c.layers <= 0 || c.B <= 0 || c.d <= 0 || c.F <= 0 || c.H <= 0 || c.Hkv <= 0 || c.H % c.Hkv || c.hd <= 0 ||
-      c.hd > 128 || c.hd * c.H != c.d || c.n_prefix < 0 || c.act < 0 || c.act > 3 || (c.rms && !c.pre_norm))
+      c.hd > 128 || c.hd * c.H != c.d || c.n_prefix < 0 || c.cache_rows <= 0 || c.act < 0 || c.act > 3 || (c.rms && !c.pre_norm))
     return DZ_ERR_ARG;
   if (c.B > SK_MAX_ROWS || (c.d >> 3) > 2048) return DZ_ERR_TOO_LARGE;
   if ((c.d & 7) || (c.F & 7) || (c.hd & 7) || (c.ld_seq & 7) || (c.ld_row & 7) || (c.n_prefix && (c.ld_prefix & 7)))
@@ -139,11 +140,14 @@ extern "C" void dz_decode_plan_free(void* plan) { delete static_cast<DecodePlan*
 // row t of every sequence is written, columns [pad_left, t] are attended to.  Asynchronous on `stream`.
 extern "C" int dz_decode_step(const void* plan, const void* const* k_cache, const void* const* v_cache, int t,
                               const int* pad_left, cudaStream_t stream) {
-  if (!plan || !k_cache || !v_cache || t < 0) return DZ_ERR_ARG;
+  if (!plan || !k_cache || !v_cache) return DZ_ERR_ARG;
   const DecodePlan& p = *static_cast<const DecodePlan*>(plan);
   const DzDecodeConfig& c = p.c;
-  if (sizeof(float) * ((size_t)c.n_prefix + t + 1) > 160 * 1024) return DZ_ERR_TOO_LARGE;   // as dz_decode_attn
+  if (t < 0 || t >= c.cache_rows) return DZ_ERR_ARG;            // row t of every sequence is written
+  if ((long long)c.n_prefix + t + 1 > DA_MAX_KEYS) return DZ_ERR_TOO_LARGE;
   if (c.rope_n_pos && c.n_prefix + t >= c.rope_n_pos) return DZ_ERR_ARG;
+  for (int i = 0; i < c.layers; ++i)
+    if (!k_cache[i] || !v_cache[i]) return DZ_ERR_ARG;
   const int n_qkv = (c.H + 2 * c.Hkv) * c.hd;
   auto B16 = [](const void* q) { return static_cast<const __nv_bfloat16*>(q); };
   bool first = true;
@@ -167,7 +171,6 @@ extern "C" int dz_decode_step(const void* plan, const void* const* k_cache, cons
   };
   for (int i = 0; i < c.layers; ++i) {
     const LayerPlan& l = p.layers[i];
-    if (!k_cache[i] || !v_cache[i]) return DZ_ERR_ARG;
     int rc = DZ_OK;
     if (c.pre_norm) rc = norm(c.h, l.w.ln1_w, l.w.ln1_b, c.xn);
     if (!rc) rc = gemm(l.qkv, c.pre_norm ? p.x_xn : p.x_h, l.w.qkv_w, c.pre_norm ? c.xn : c.h, c.qkv, n_qkv, c.d, l.w.qkv_b, nullptr, 0);

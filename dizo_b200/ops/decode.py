@@ -81,7 +81,7 @@ class _Layer(ctypes.Structure):
 
 class _Config(ctypes.Structure):
     _fields_ = ([(n, ctypes.c_int) for n in ("layers", "B", "d", "F", "H", "Hkv", "hd", "n_prefix", "rms", "pre_norm",
-                                             "act", "rope_n_pos")] +
+                                             "act", "rope_n_pos", "cache_rows")] +
                 [("eps", ctypes.c_float), ("scale", ctypes.c_float)] +
                 [(n, ctypes.c_longlong) for n in ("ld_prefix", "ld_seq", "ld_row")] +
                 [(n, ctypes.c_void_p) for n in ("rope_cs", "h", "h2", "xn", "qkv", "ctx", "f", "err")])
@@ -94,10 +94,11 @@ class DecodePlan:
     """All blocks of one decoding step as a single native call (``csrc/decode_step.cu``).
 
     ``layers``: per block a dict of the names in ``_LAYER_FIELDS`` -> bf16 CUDA tensor or None; the plan keeps them and
-    its workspaces alive.  ``h`` [B, d] holds the embedded tokens before :meth:`step` and the last block's output after."""
+    its workspaces alive.  ``h`` [B, d] holds the embedded tokens before :meth:`step` and the last block's output after.
+    The caches are bf16 [B, cache_rows, d] per layer; a step at or past ``cache_rows`` is refused."""
 
     def __init__(self, layers: list[dict], B: int, d: int, F: int, H: int, Hkv: int, act: int, rms: bool,
-                 pre_norm: bool, eps: float, ld_seq: int, ld_row: int, rope: torch.Tensor | None = None):
+                 pre_norm: bool, eps: float, cache_rows: int, rope: torch.Tensor | None = None):
         self._handle = ctypes.c_void_p()
         self._free = _lib.lib().dz_decode_plan_free      # held here: module globals may be gone when the plan is
         dev = layers[0]["qkv_w"].device
@@ -106,6 +107,7 @@ class DecodePlan:
         self.h, self._ws = ws(d), [ws(d), ws(d), ws((H + 2 * Hkv) * hd), ws(d), ws(F)]
         self._keep = (layers, rope)
         self._kernels = 7 * len(layers)
+        self._cache_rows = cache_rows
         pk = layers[0].get("prefix_k")
         for w in layers:
             for n in _LAYER_FIELDS:
@@ -115,15 +117,19 @@ class DecodePlan:
         p = lambda t: _lib.ptr(t).value                                               # noqa: E731
         cfg = _Config(layers=len(layers), B=B, d=d, F=F, H=H, Hkv=Hkv, hd=hd, n_prefix=0 if pk is None else pk.shape[0],
                       rms=int(rms), pre_norm=int(pre_norm), act=act, rope_n_pos=0 if rope is None else rope.shape[0],
-                      eps=eps, scale=hd ** -0.5, ld_prefix=0 if pk is None else pk.stride(0), ld_seq=ld_seq,
-                      ld_row=ld_row, rope_cs=p(rope), h=p(self.h), h2=p(self._ws[0]), xn=p(self._ws[1]),
-                      qkv=p(self._ws[2]), ctx=p(self._ws[3]), f=p(self._ws[4]), err=p(_lib.err_word(dev)))
+                      eps=eps, scale=hd ** -0.5, ld_prefix=0 if pk is None else pk.stride(0),
+                      ld_seq=cache_rows * d, ld_row=d, cache_rows=cache_rows, rope_cs=p(rope), h=p(self.h),
+                      h2=p(self._ws[0]), xn=p(self._ws[1]), qkv=p(self._ws[2]), ctx=p(self._ws[3]), f=p(self._ws[4]),
+                      err=p(_lib.err_word(dev)))
         _lib.check(_lib.lib().dz_decode_plan_create(ctypes.byref(cfg), arr, ctypes.byref(self._handle)),
                    "dz_decode_plan_create")
 
     def caches(self, k: list[torch.Tensor], v: list[torch.Tensor]):
         """Pointer arrays of the per-layer caches for :meth:`step` (kept by the caller beside the tensors)."""
-        n = len(k)
+        n, shape = len(self._keep[0]), (self.h.shape[0], self._cache_rows, self.h.shape[1])
+        assert len(k) == n == len(v)
+        for t in (*k, *v):
+            assert t.shape == shape and t.is_contiguous() and t.dtype == torch.bfloat16 and t.device == self.h.device
         return tuple((ctypes.c_void_p * n)(*[_lib.ptr(t).value for t in ts]) for ts in (k, v))
 
     def step(self, caches, t: int, pad_left: torch.Tensor) -> torch.Tensor:

@@ -64,3 +64,38 @@ def test_checked_store_build_reports_and_skips_unregistered_stores():
     res = subprocess.run([sys.executable, "-c", SCRIPT], env=env, capture_output=True, text=True, timeout=900, cwd=ROOT)
     assert res.returncode == 0 and "CLEAN" in res.stdout and "REPORTED" in res.stdout, \
         (res.stdout[-3000:], res.stderr[-3000:])
+
+
+DECODE_SCRIPT = textwrap.dedent('''
+    import torch
+    from dizo_b200.models.generate import _Decoder, generate
+    from dizo_b200.models.opt import OPTModel, make_batch, preset
+    from dizo_b200.ops import _lib
+    assert _lib.DEBUG_BOUNDS
+    m = OPTModel(preset("opt-125m", num_hidden_layers=2), "cuda", torch.bfloat16).init_random_fast(0)
+    ids = torch.arange(4, 28).view(2, 12)
+    generate(m, ids, max_new_tokens=4, do_sample=True, top_p=0.9, seed=1)
+    generate(m, ids, max_new_tokens=4, num_beams=2)
+    _lib.check_device_errors()
+    batch = make_batch(ids).to("cuda")
+    dec = _Decoder(m, 2, 16)
+    dec.prefill(batch)
+    tok = torch.full((2,), 7, dtype=torch.int32, device="cuda")
+    dec.step(tok, tok + 7, batch.pad_left)
+    _lib.check_device_errors()
+    print("CLEAN")
+    _lib.forget(dec.k[1])                           # the append into this cache must be skipped and reported
+    before = dec.k[1].clone()
+    dec.step(tok, tok + 8, batch.pad_left)
+    bad = _lib.debug_violations()
+    assert len(bad) == 1 and bad[0][0] == "decode" and bad[0][1] == 2 * 768, bad
+    assert torch.equal(before, dec.k[1])
+    print("REPORTED", bad)
+''')
+
+
+def test_checked_store_build_sees_the_cache_append():
+    env = dict(os.environ, DIZO_DEBUG_BOUNDS="1", PYTHONPATH=ROOT)
+    res = subprocess.run([sys.executable, "-c", DECODE_SCRIPT], env=env, capture_output=True, text=True, timeout=900, cwd=ROOT)
+    assert res.returncode == 0 and "CLEAN" in res.stdout and "REPORTED" in res.stdout, \
+        (res.stdout[-3000:], res.stderr[-3000:])

@@ -63,6 +63,22 @@ def test_native_step_equals_block_by_block(name, B, L):
     assert ((a - b).norm() / b.norm()).item() < 2 * 2.0 ** -8
 
 
+@pytest.mark.parametrize("name", ["opt", "llama"])
+def test_step_past_the_caches_is_refused(name):
+    m = _models()[name]().init_random_fast(3, std=0.05)
+    batch = make_batch(torch.arange(4, 16).view(2, 6)).to("cuda")
+    dec = _Decoder(m, 2, 7)
+    dec.prefill(batch)
+    tok = torch.full((2,), 7, dtype=torch.int32, device="cuda")
+    pos = torch.full((2,), 8, dtype=torch.int32, device="cuda")
+    dec.step(tok, pos, batch.pad_left)
+    before = [x.clone() for x in dec.k + dec.v]
+    with pytest.raises((_lib.KernelError, IndexError)):
+        dec.step(tok, pos + 1, batch.pad_left)
+    _lib.check_device_errors()
+    assert dec.len == 7 and all(torch.equal(x, y) for x, y in zip(before, dec.k + dec.v))
+
+
 @pytest.mark.parametrize("V", [7, 512, 2049, 32000, 51200])
 @pytest.mark.parametrize("top_k,top_p", [(None, None), (40, None), (None, 0.9), (300, 0.6)])
 def test_sampler_forms_agree(V, top_k, top_p):
