@@ -75,7 +75,7 @@ class _Decoder:
             if m.use_lora and not m._merge_buf["per_layer"]:
                 self.native = False                            # one merge buffer for all blocks: merged anew per block
                 return
-        if not layers:
+        if not layers or self.k[0].shape[0] > decode_ops.MAX_STEP_ROWS:
             self.native = False
             return
         B, max_len, d = self.k[0].shape
@@ -105,6 +105,8 @@ class _Decoder:
             self.k[i] = self.k[i].index_select(0, index)
             self.v[i] = self.v[i].index_select(0, index)
         self._caches = None
+        if self.plan is not None and self.plan.h.shape[0] != index.shape[0]:
+            self.plan = None                                   # another number of sequences: its workspaces do not fit
 
     def step(self, tokens: torch.Tensor, positions: torch.Tensor, pad_left: torch.Tensor) -> torch.Tensor:
         """tokens, positions: int32 [B]; returns the next-token logits [B, V] (fp32)."""
@@ -116,6 +118,7 @@ class _Decoder:
         if self.native:
             if self._caches is None:
                 self._caches = self.plan.caches(self.k, self.v)
+            assert h.shape == self.plan.h.shape and (pad_left is None or pad_left.shape[0] == h.shape[0])
             self.plan.h.copy_(h)
             h = self.plan.step(self._caches, t, pad_left)
             self.len = t + 1

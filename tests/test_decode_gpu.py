@@ -79,6 +79,24 @@ def test_step_past_the_caches_is_refused(name):
     assert dec.len == 7 and all(torch.equal(x, y) for x, y in zip(before, dec.k + dec.v))
 
 
+def test_step_after_a_reorder_to_fewer_sequences():
+    m = _models()["opt"]().init_random_fast(3, std=0.05)
+    batch = make_batch(torch.arange(4, 28).view(4, 6)).to("cuda")
+    tok = torch.full((4,), 7, dtype=torch.int32, device="cuda")
+    pos = torch.full((4,), 8, dtype=torch.int32, device="cuda")
+    index = torch.tensor([2], device="cuda")
+    out = []
+    for native in (True, False):
+        dec = _Decoder(m, 4, 16)
+        dec.native = native
+        dec.prefill(batch)
+        dec.step(tok, pos, batch.pad_left)
+        dec.reorder(index)
+        out.append(dec.step(tok[:1], pos[:1] + 1, batch.pad_left[index]))
+    _lib.check_device_errors()
+    assert ((out[0] - out[1]).norm() / out[1].norm()).item() < 2 * 2.0 ** -8
+
+
 @pytest.mark.parametrize("V", [7, 512, 2049, 32000, 51200])
 @pytest.mark.parametrize("top_k,top_p", [(None, None), (40, None), (None, 0.9), (300, 0.6)])
 def test_sampler_forms_agree(V, top_k, top_p):
