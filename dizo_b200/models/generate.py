@@ -110,16 +110,27 @@ class _Decoder:
 
     def step(self, tokens: torch.Tensor, positions: torch.Tensor, pad_left: torch.Tensor) -> torch.Tensor:
         """tokens, positions: int32 [B]; returns the next-token logits [B, V] (fp32)."""
+        return self.advance(self.embed(tokens, positions), pad_left)
+
+    def embed(self, tokens: torch.Tensor, positions: torch.Tensor) -> torch.Tensor:
+        """The first part of a step: what :meth:`advance` sends through the blocks."""
         m = self.m
-        t = self.len
         h = m.decode_embed(tokens, positions, m._resolver(-1, None, None, 0))
         if self.native and self.plan is None:
             self._build_plan()
         if self.native:
             if self._caches is None:
                 self._caches = self.plan.caches(self.k, self.v)
-            assert h.shape == self.plan.h.shape and (pad_left is None or pad_left.shape[0] == h.shape[0])
-            self.plan.h.copy_(h)
+            assert h.shape == self.plan.h.shape
+            return self.plan.h.copy_(h)
+        return h
+
+    def advance(self, h: torch.Tensor, pad_left: torch.Tensor) -> torch.Tensor:
+        """The blocks of one step, from :meth:`embed`'s result to the logits."""
+        m = self.m
+        t = self.len
+        if self.native:
+            assert pad_left is None or pad_left.shape[0] == h.shape[0]
             h = self.plan.step(self._caches, t, pad_left)
             self.len = t + 1
             return _head_logits(m, h)
@@ -330,7 +341,9 @@ def _make_decoder(model, B: int, max_len: int) -> _Decoder:
 def _extend(dec: _Decoder, logits: torch.Tensor, out: List[List[int]], pos: torch.Tensor, pad_left: torch.Tensor,
             max_new_tokens: int, eos: set, pad_token_id: int, **sampling) -> None:
     """Greedy / sampled continuation of the rows of ``out`` on CUDA.  A token stays on the device between the sampling
-    kernel and the next step, which is queued before the host looks at the token: the host's part runs beside the step."""
+    kernel and the next step.  Without end-of-sequence ids the step is queued before the host looks at the token: the host's
+    part runs beside it.  With them only its embedding is: the blocks follow once a row is known to go on, so that no
+    step is left on the stream behind the last token."""
     dev = logits.device
     B = len(out)
     done = torch.zeros(B, dtype=torch.int32, device=dev)
@@ -342,15 +355,23 @@ def _extend(dec: _Decoder, logits: torch.Tensor, out: List[List[int]], pos: torc
         nxt = decode_ops.sample_step(logits, offset=t, done=done, eos=eos_dev, pad_id=pad_token_id, **sampling)
         host[t].copy_(nxt, non_blocking=True)
         ready.record()
-        if t + 1 < max_new_tokens:
-            logits = dec.step(nxt, pos, pad_left)
+        more = t + 1 < max_new_tokens
+        if more:
+            h = dec.embed(nxt, pos)
             pos = pos + 1
+            if not eos:
+                logits = dec.advance(h, pad_left)
         ready.synchronize()
-        for i, tok in enumerate(host[t].tolist()):
+        toks = host[t].tolist()
+        over = [e or tok in eos for e, tok in zip(ended, toks)]
+        more = more and not all(over)
+        if more and eos:
+            logits = dec.advance(h, pad_left)
+        for i, tok in enumerate(toks):
             if not ended[i]:
                 out[i].append(tok)
-                ended[i] = tok in eos
-        if all(ended):
+        ended = over
+        if not more:
             break
 
 

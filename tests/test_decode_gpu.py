@@ -141,3 +141,20 @@ def test_generate_stops_rows_at_an_end_of_sequence_id(sample):
             end = next((i + 1 for i in range(prompt, len(row)) if row[i] in stop), len(row))
             assert out == row[:end]
     assert generate(m, ids, mask, max_new_tokens=0) == [r[k.bool()].tolist() for r, k in zip(ids, mask)]
+
+
+@pytest.mark.parametrize("name", ["opt", "llama"])
+def test_generate_queues_no_step_behind_the_last_token(name, monkeypatch):
+    m = _models()[name]().init_random_fast(3, std=0.05)
+    ids = torch.randint(4, 500, (2, 20), generator=torch.Generator().manual_seed(4))
+    steps = []
+    step = decode_ops.DecodePlan.step
+    monkeypatch.setattr(decode_ops.DecodePlan, "step", lambda self, *a: (steps.append(1), step(self, *a))[1])
+    kw = dict(max_new_tokens=9, do_sample=True, seed=3)
+    free = generate(m, ids, **kw)
+    assert len(steps) == 8 and all(len(r) == 29 for r in free)
+    stop = {r[20 + i] for i, r in enumerate(free)}                 # the rows end with their first and second token at latest
+    del steps[:]
+    got = generate(m, ids, eos_token_id=sorted(stop), **kw)
+    assert len(steps) == max(len(r) for r in got) - 21
+    assert all(r == f[:len(r)] and r[-1] in stop for r, f in zip(got, free))
