@@ -487,10 +487,3 @@ extern "C" int dz_sample_step(const float* logits, long long ld, int rows, int V
   }
   return cuda_rc(cudaGetLastError());
 }
-
-extern "C" int dz_sample_topk_topp(const float* logits, long long ld, int rows, int V, float temperature,
-                                   int top_k, float top_p, int do_sample, unsigned long long seed,
-                                   unsigned long long offset, int* out, cudaStream_t stream) {
-  return dz_sample_step(logits, ld, rows, V, temperature, top_k, top_p, do_sample, seed, offset, nullptr, nullptr, 0, 0,
-                        out, stream);
-}
