@@ -346,6 +346,7 @@ def _extend(dec: _Decoder, logits: torch.Tensor, out: List[List[int]], pos: torc
     step is left on the stream behind the last token."""
     dev = logits.device
     B = len(out)
+    eos = {e for e in eos if 0 <= e < logits.shape[1]}         # no other id can be drawn
     done = torch.zeros(B, dtype=torch.int32, device=dev)
     eos_dev = torch.tensor(sorted(eos), dtype=torch.int32).to(dev) if eos else None
     host = torch.empty((max_new_tokens, B), dtype=torch.int32, pin_memory=True)

@@ -158,3 +158,9 @@ def test_generate_queues_no_step_behind_the_last_token(name, monkeypatch):
     got = generate(m, ids, eos_token_id=sorted(stop), **kw)
     assert len(steps) == max(len(r) for r in got) - 21
     assert all(r == f[:len(r)] and r[-1] in stop for r, f in zip(got, free))
+
+
+def test_generate_takes_end_of_sequence_ids_outside_the_vocabulary():
+    m = _models()["opt"]().init_random_fast(3, std=0.05)
+    ids = torch.arange(4, 16).view(2, 6)
+    assert generate(m, ids, max_new_tokens=3, eos_token_id=[-1, 520, 2 ** 40]) == generate(m, ids, max_new_tokens=3)
