@@ -53,6 +53,8 @@ class _Decoder:
     first step of a run); CPU tensors, more than ``MAX_STEP_ROWS`` sequences and LoRA operands that share one merge buffer
     go block by block through ``model.decode_block``."""
 
+    plan, _caches, native = None, None, False      # sharded decoders, with a step of their own, leave these as they are
+
     def __init__(self, model: OPTModel, B: int, max_len: int):
         self.m = model
         cfg = model.config
@@ -63,7 +65,6 @@ class _Decoder:
         self.k = [torch.empty(B, max_len, d, dtype=dt, device=dev) for _ in range(cfg.num_hidden_layers)]
         self.v = [torch.empty(B, max_len, d, dtype=dt, device=dev) for _ in range(cfg.num_hidden_layers)]
         self.len = 0
-        self.plan, self._caches = None, None
         self.native = (dev.type == "cuda" and dt == torch.bfloat16 and B <= decode_ops.MAX_STEP_ROWS
                        and getattr(type(model), "step_layer", None) is not None)
 

@@ -1,7 +1,10 @@
 """Host side of decoding: the caches of a run."""
+from types import SimpleNamespace
+
+import pytest
 import torch
 
-from dizo_b200.models.generate import _Decoder
+from dizo_b200.models.generate import _Decoder, _PPDecoder, _TPDecoder
 from dizo_b200.models.opt import OPTConfig, OPTModel
 
 
@@ -16,3 +19,15 @@ def test_each_cache_owns_its_memory():
         assert len({t.untyped_storage().data_ptr() for t in tensors}) == len(tensors) == 6
         assert all(t.untyped_storage().nbytes() == 4 * 10 * 32 * 4 for t in tensors)
         dec.reorder(torch.tensor([1, 0, 3, 3]))
+
+
+@pytest.mark.parametrize("cls", [_Decoder, _TPDecoder, _PPDecoder])
+def test_every_decoder_reorders_its_caches(cls):
+    m = SimpleNamespace(config=SimpleNamespace(hidden_size=16, num_hidden_layers=2), device=torch.device("cpu"),
+                        dtype=torch.float32, tp=2, lo=0, hi=2)
+    dec = cls(m, 3, 5)
+    for i, t in enumerate(dec.k + dec.v):
+        t.copy_(torch.arange(3.0).view(3, 1, 1) + 10 * i)
+    dec.reorder(torch.tensor([2, 0]))
+    for i, t in enumerate(dec.k + dec.v):
+        assert t.shape[:2] == (2, 5) and t[:, 0, 0].tolist() == [10 * i + 2, 10 * i]
