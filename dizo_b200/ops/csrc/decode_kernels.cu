@@ -455,6 +455,8 @@ extern "C" int dz_decode_attn(const void* q, long long ldq, const void* kc, cons
   if (!q || !kc || !vc || !out || B <= 0 || H <= 0 || kv_len <= 0) return DZ_ERR_ARG;
   if (hd > 128 || (hd & 7) || (ld_row & 7) || (ld_seq & 7) || (n_prefix > 0 && (!pk || !pv || (ldp & 7))))
     return DZ_ERR_ARG;
+  for (const void* rows : {kc, vc, pk, pv})                       // read in 16-byte vectors
+    if (reinterpret_cast<uintptr_t>(rows) & 15) return DZ_ERR_ALIGN;
   if ((long long)n_prefix + kv_len > DA_MAX_KEYS) return DZ_ERR_TOO_LARGE;
   DecodeAttnArgs a{};
   a.q = (const __nv_bfloat16*)q; a.ldq = ldq;

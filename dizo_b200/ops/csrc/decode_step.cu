@@ -146,8 +146,10 @@ extern "C" int dz_decode_step(const void* plan, const void* const* k_cache, cons
   if (t < 0 || t >= c.cache_rows) return DZ_ERR_ARG;            // row t of every sequence is written
   if ((long long)c.n_prefix + t + 1 > DA_MAX_KEYS) return DZ_ERR_TOO_LARGE;
   if (c.rope_n_pos && c.n_prefix + t >= c.rope_n_pos) return DZ_ERR_ARG;
-  for (int i = 0; i < c.layers; ++i)
+  for (int i = 0; i < c.layers; ++i) {
     if (!k_cache[i] || !v_cache[i]) return DZ_ERR_ARG;
+    if (!al16(k_cache[i]) || !al16(v_cache[i])) return DZ_ERR_ALIGN;
+  }
   const int n_qkv = (c.H + 2 * c.Hkv) * c.hd;
   auto B16 = [](const void* q) { return static_cast<const __nv_bfloat16*>(q); };
   bool first = true;

@@ -26,6 +26,11 @@ def decode_attention(q, k_cache, v_cache, kv_len, n_heads, pad_left=None, prefix
     npre = prefix_k.shape[0] if prefix_k is not None else 0
     assert q.stride(-1) == 1 and k_cache.stride(-1) == 1 and v_cache.stride(-1) == 1
     assert k_cache.stride() == v_cache.stride()
+    # the kernel reads rows in 16-byte vectors: rows that start elsewhere are copied
+    if (k_cache.data_ptr() | v_cache.data_ptr()) & 15:
+        k_cache, v_cache = (t.clone(memory_format=torch.contiguous_format) for t in (k_cache, v_cache))
+    if prefix_k is not None and (prefix_k.data_ptr() | prefix_v.data_ptr()) & 15:
+        prefix_k, prefix_v = (t.clone(memory_format=torch.contiguous_format) for t in (prefix_k, prefix_v))
     rc = _lib.lib().dz_decode_attn(
         _lib.ptr(q), ll(q.stride(0)), _lib.ptr(k_cache), _lib.ptr(v_cache), ll(k_cache.stride(0)),
         ll(k_cache.stride(1)), _lib.ptr(prefix_k), _lib.ptr(prefix_v),

@@ -1,4 +1,6 @@
 """Decoding kernels: native decoding steps against the block-by-block path, the sampler's two forms."""
+import math
+
 import pytest
 import torch
 
@@ -95,6 +97,23 @@ def test_step_after_a_reorder_to_fewer_sequences():
         out.append(dec.step(tok[:1], pos[:1] + 1, batch.pad_left[index]))
     _lib.check_device_errors()
     assert ((out[0] - out[1]).norm() / out[1].norm()).item() < 2 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("shift", [0, 4, 1])
+def test_decode_attention_over_rows_off_a_16_byte_boundary(shift):
+    """Caches and prefix rows may start anywhere: the values are those of the aligned ones, bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(shift)
+    B, n, H, hd, P = 2, 37, 3, 64, 5
+
+    def rows(*shape):
+        flat = torch.randn(math.prod(shape) + shift, device="cuda", generator=g).bfloat16()
+        return flat[shift:].view(shape)
+
+    q, k, v, pk, pv = rows(B, H * hd), rows(B, n, H * hd), rows(B, n, H * hd), rows(P, H * hd), rows(P, H * hd)
+    y = decode_ops.decode_attention(q, k, v, n - 1, H, None, pk, pv)
+    ref = decode_ops.decode_attention(q, k.clone(), v.clone(), n - 1, H, None, pk.clone(), pv.clone())
+    _lib.check_device_errors()
+    assert torch.equal(y, ref)
 
 
 @pytest.mark.parametrize("V", [7, 512, 2049, 32000, 51200])
