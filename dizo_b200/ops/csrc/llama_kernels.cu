@@ -17,9 +17,10 @@
 
 namespace dz {
 
-constexpr int RMS_MAXV = 4;  // uint4 (8 bf16) per thread held in registers
+constexpr int RMS_MAXV = 4;  // most uint4 (8 bf16) per thread held in registers
 
-template <int THREADS>
+// NV and AHEAD as in layernorm_kernel (norm_embed.cu).
+template <int THREADS, int NV, bool AHEAD>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w,
                __nv_bfloat16* __restrict__ y, long long ldy, int d, float eps) {
@@ -29,10 +30,10 @@ rmsnorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w,
   const long long row = blockIdx.x;
   const int nvec = d >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * ldx);
-  uint4 v[RMS_MAXV];
+  uint4 v[NV];
   float sq = 0.f;
 #pragma unroll
-  for (int i = 0; i < RMS_MAXV; ++i) {
+  for (int i = 0; i < NV; ++i) {
     const int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
       v[i] = __ldcg(xr + idx);
@@ -52,18 +53,20 @@ rmsnorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w,
   const float rstd = rsqrtf(tot / d + eps);
   uint4* yr = reinterpret_cast<uint4*>(y + row * ldy);
   const uint4* wr = reinterpret_cast<const uint4*>(w);
-  // coherent loads: the sweep right in front of this kernel may have written w (pdl.cuh).  All before the first store,
-  // which they may not pass.
-  uint4 wv[RMS_MAXV];
+  // coherent loads: the sweep right in front of this kernel may have written w (pdl.cuh)
+  uint4 wv[NV];
+  if (AHEAD) {
 #pragma unroll
-  for (int i = 0; i < RMS_MAXV; ++i) {
-    const int idx = threadIdx.x + i * THREADS;
-    if (idx < nvec) wv[i] = __ldca(wr + idx);
+    for (int i = 0; i < NV; ++i) {
+      const int idx = threadIdx.x + i * THREADS;
+      if (idx < nvec) wv[i] = __ldca(wr + idx);
+    }
   }
 #pragma unroll
-  for (int i = 0; i < RMS_MAXV; ++i) {
+  for (int i = 0; i < NV; ++i) {
     const int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
+      if (!AHEAD) wv[i] = wr[idx];
       uint4 o;
       o.x = pack_bf16x2(bf16_lo(v[i].x) * rstd * bf16_lo(wv[i].x), bf16_hi(v[i].x) * rstd * bf16_hi(wv[i].x));
       o.y = pack_bf16x2(bf16_lo(v[i].y) * rstd * bf16_lo(wv[i].y), bf16_hi(v[i].y) * rstd * bf16_hi(wv[i].y));
@@ -132,16 +135,27 @@ silu_mul_kernel(const __nv_bfloat16* __restrict__ gu, long long ld, __nv_bfloat1
   }
 }
 
-int rmsnorm_launch(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, __nv_bfloat16* y, long long ldy,
-                   long long rows, int d, float eps, bool dependent, cudaStream_t stream) {
+template <bool AHEAD>
+static int rmsnorm_nv(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, __nv_bfloat16* y, long long ldy,
+                      long long rows, int d, float eps, bool dependent, cudaStream_t stream) {
   const int nvec = d >> 3;
   auto launch = [&](auto kern, int threads) {
     return cuda_rc(pdl_launch(kern, dim3((unsigned)rows), threads, 0, stream, 1, dependent, x, ldx, w, y, ldy, d, eps));
   };
-  if (nvec <= 128 * RMS_MAXV) return launch(rmsnorm_kernel<128>, 128);
-  if (nvec <= 256 * RMS_MAXV) return launch(rmsnorm_kernel<256>, 256);
-  if (nvec <= 512 * RMS_MAXV) return launch(rmsnorm_kernel<512>, 512);
+  if (nvec <= 128) return launch(rmsnorm_kernel<128, 1, AHEAD>, 128);
+  if (nvec <= 256) return launch(rmsnorm_kernel<128, 2, AHEAD>, 128);
+  if (nvec <= 384) return launch(rmsnorm_kernel<128, 3, AHEAD>, 128);
+  if (nvec <= 128 * RMS_MAXV) return launch(rmsnorm_kernel<128, RMS_MAXV, AHEAD>, 128);
+  if (nvec <= 768) return launch(rmsnorm_kernel<256, 3, AHEAD>, 256);
+  if (nvec <= 256 * RMS_MAXV) return launch(rmsnorm_kernel<256, RMS_MAXV, AHEAD>, 256);
+  if (nvec <= 512 * RMS_MAXV) return launch(rmsnorm_kernel<512, RMS_MAXV, AHEAD>, 512);
   return DZ_ERR_TOO_LARGE;
+}
+
+int rmsnorm_launch(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, __nv_bfloat16* y, long long ldy,
+                   long long rows, int d, float eps, bool dependent, cudaStream_t stream) {
+  return rows <= 8LL * sm_count() ? rmsnorm_nv<true>(x, ldx, w, y, ldy, rows, d, eps, dependent, stream)
+                                  : rmsnorm_nv<false>(x, ldx, w, y, ldy, rows, d, eps, dependent, stream);
 }
 
 static inline bool lk_al16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }

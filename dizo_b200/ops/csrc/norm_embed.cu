@@ -15,9 +15,13 @@
 
 namespace dz {
 
-constexpr int LN_MAXV = 4;  // uint4 (8 bf16) per thread held in registers
+constexpr int LN_MAXV = 4;  // most uint4 (8 bf16) per thread held in registers
 
-template <int THREADS>
+// One CTA per row, NV = ceil(d / (8 THREADS)) vectors a thread.  AHEAD: all of w and b is loaded before the first store
+// (coherent loads may not pass it), which shortens the row; without, they come vector by vector and 40 registers instead of
+// 64 let half as many CTAs again share an SM.  Back-to-back launches, us, ahead / not: 1024 x 2560 3.3 / 4.1, 1024 x 4096
+// 3.9 / 4.4; 8192 x 768 11.3 / 9.4, 4096 x 5120 17.1 / 14.9, 8192 x 5120 37.6 / 31.9.
+template <int THREADS, int NV, bool AHEAD>
 __global__ void __launch_bounds__(THREADS)
 layernorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* b,
                  __nv_bfloat16* __restrict__ y, long long ldy, int d, float eps) {
@@ -28,10 +32,10 @@ layernorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, 
   const long long row = blockIdx.x;
   const int nvec = d >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * ldx);
-  uint4 v[LN_MAXV];
+  uint4 v[NV];
   float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < LN_MAXV; ++i) {
+  for (int i = 0; i < NV; ++i) {
     int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
       v[i] = __ldcg(xr + idx);
@@ -57,7 +61,7 @@ layernorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, 
   const float mean = block_sum(sum) / d;
   float sq = 0.f;
 #pragma unroll
-  for (int i = 0; i < LN_MAXV; ++i) {
+  for (int i = 0; i < NV; ++i) {
     int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
       float f[8] = {bf16_lo(v[i].x), bf16_hi(v[i].x), bf16_lo(v[i].y), bf16_hi(v[i].y),
@@ -73,21 +77,23 @@ layernorm_kernel(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, 
   uint4* yr = reinterpret_cast<uint4*>(y + row * ldy);
   const uint4* wr = reinterpret_cast<const uint4*>(w);
   const uint4* br = reinterpret_cast<const uint4*>(b);
-  // coherent loads: the sweep right in front of this kernel may have written w and b (pdl.cuh).  All before the first
-  // store, which they may not pass.
-  uint4 wv[LN_MAXV], bv[LN_MAXV];
+  // coherent loads: the sweep right in front of this kernel may have written w and b (pdl.cuh)
+  uint4 wv[NV], bv[NV];
+  if (AHEAD) {
 #pragma unroll
-  for (int i = 0; i < LN_MAXV; ++i) {
-    const int idx = threadIdx.x + i * THREADS;
-    if (idx < nvec) {
-      wv[i] = __ldca(wr + idx);
-      bv[i] = __ldca(br + idx);
+    for (int i = 0; i < NV; ++i) {
+      const int idx = threadIdx.x + i * THREADS;
+      if (idx < nvec) {
+        wv[i] = __ldca(wr + idx);
+        bv[i] = __ldca(br + idx);
+      }
     }
   }
 #pragma unroll
-  for (int i = 0; i < LN_MAXV; ++i) {
+  for (int i = 0; i < NV; ++i) {
     int idx = threadIdx.x + i * THREADS;
     if (idx < nvec) {
+      if (!AHEAD) { wv[i] = wr[idx]; bv[i] = br[idx]; }
       uint4 o;
       o.x = pack_bf16x2((bf16_lo(v[i].x) - mean) * rstd * bf16_lo(wv[i].x) + bf16_lo(bv[i].x),
                         (bf16_hi(v[i].x) - mean) * rstd * bf16_hi(wv[i].x) + bf16_hi(bv[i].x));
@@ -165,17 +171,30 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ src, long long lds, const i
     if (DZ_STORE_OK(orow + i, 16)) orow[i] = sr[i];
 }
 
-int layernorm_launch(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* b,
-                     __nv_bfloat16* y, long long ldy, long long rows, int d, float eps, bool dependent,
-                     cudaStream_t stream) {
+template <bool AHEAD>
+static int layernorm_nv(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* b,
+                        __nv_bfloat16* y, long long ldy, long long rows, int d, float eps, bool dependent,
+                        cudaStream_t stream) {
   const int nvec = d >> 3;
   auto launch = [&](auto kern, int threads) {
     return cuda_rc(pdl_launch(kern, dim3((unsigned)rows), threads, 0, stream, 1, dependent, x, ldx, w, b, y, ldy, d, eps));
   };
-  if (nvec <= 128 * LN_MAXV) return launch(layernorm_kernel<128>, 128);
-  if (nvec <= 256 * LN_MAXV) return launch(layernorm_kernel<256>, 256);
-  if (nvec <= 512 * LN_MAXV) return launch(layernorm_kernel<512>, 512);
+  if (nvec <= 128) return launch(layernorm_kernel<128, 1, AHEAD>, 128);
+  if (nvec <= 256) return launch(layernorm_kernel<128, 2, AHEAD>, 128);
+  if (nvec <= 384) return launch(layernorm_kernel<128, 3, AHEAD>, 128);
+  if (nvec <= 128 * LN_MAXV) return launch(layernorm_kernel<128, LN_MAXV, AHEAD>, 128);
+  if (nvec <= 768) return launch(layernorm_kernel<256, 3, AHEAD>, 256);
+  if (nvec <= 256 * LN_MAXV) return launch(layernorm_kernel<256, LN_MAXV, AHEAD>, 256);
+  if (nvec <= 512 * LN_MAXV) return launch(layernorm_kernel<512, LN_MAXV, AHEAD>, 512);
   return DZ_ERR_TOO_LARGE;
+}
+
+int layernorm_launch(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w, const __nv_bfloat16* b,
+                     __nv_bfloat16* y, long long ldy, long long rows, int d, float eps, bool dependent,
+                     cudaStream_t stream) {
+  // ahead while every 128-thread CTA with its 64 registers a thread is resident at once
+  return rows <= 8LL * sm_count() ? layernorm_nv<true>(x, ldx, w, b, y, ldy, rows, d, eps, dependent, stream)
+                                  : layernorm_nv<false>(x, ldx, w, b, y, ldy, rows, d, eps, dependent, stream);
 }
 
 }  // namespace dz

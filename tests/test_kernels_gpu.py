@@ -6,6 +6,7 @@ import torch
 
 from dizo_b200.ops import _lib, philox
 from dizo_b200.ops.attention import attention, attention_reference
+from dizo_b200.ops.llama import rmsnorm
 from dizo_b200.ops.loss import option_ce, token_logprobs, verbalizer_ce
 from dizo_b200.ops.norm import add_rows, embed, gather_rows, layernorm, opt_positions
 from dizo_b200.ops.zo import CHUNK, GammaState, ParamArena, Piece, fill_z, perturb_reference, scalar_diff
@@ -80,6 +81,24 @@ def test_layernorm(rows, d):
     y = layernorm(x, w, b)
     ref = torch.nn.functional.layer_norm(x.float(), (d,), w.float(), b.float(), 1e-5)
     assert (y.float() - ref).abs().max().item() < 4e-2
+
+
+@pytest.mark.parametrize("d", [64, 1024, 1032, 2048, 3072, 4096, 4104, 6144, 6152, 8200, 16384])
+def test_norms_over_many_rows_equal_the_same_rows_alone(d):
+    """The two forms of the norm kernels (up to 8 rows per SM, more) at every register width give the same bits."""
+    few = 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device=DEV).manual_seed(d)
+    x = (torch.randn(few + 1, d, device=DEV, generator=g) * 2 + 0.5).bfloat16()
+    w, b = (torch.randn(d, device=DEV, generator=g).bfloat16() for _ in range(2))
+    y, r = layernorm(x, w, b), rmsnorm(x, w)
+    assert torch.equal(y[:few], layernorm(x[:few], w, b)) and torch.equal(r[:few], rmsnorm(x[:few], w))
+    _sync_ok()
+    xd = x.double()
+    ref = torch.nn.functional.layer_norm(xd, (d,), w.double(), b.double(), 1e-5)
+    # one rounding to bf16 (at most 2^-8 of the value) beside the fp32 sums
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8
+    ref = xd * (xd.pow(2).mean(1, keepdim=True) + 1e-5).rsqrt() * w.double()
+    assert ((r.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8
 
 
 def test_embed_gather_add():
