@@ -1,13 +1,14 @@
 """Decoding kernels: native decoding steps against the block-by-block path, the sampler's two forms."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
 from dizo_b200.models.generate import _Decoder, generate
 from dizo_b200.models.llama import LlamaConfig, LlamaModel
 from dizo_b200.models.opt import OPTConfig, OPTModel, make_batch
-from dizo_b200.ops import _lib
+from dizo_b200.ops import _lib, philox
 from dizo_b200.ops import decode as decode_ops
 
 pytestmark = pytest.mark.gpu
@@ -116,6 +117,28 @@ def test_decode_attention_over_rows_off_a_16_byte_boundary(shift):
     assert torch.equal(y, ref)
 
 
+@pytest.mark.parametrize("V", [1024, 4096, 32768, 65536])
+def test_draw_without_filters_walks_the_mass_in_order(V):
+    """Equal logits: every probability is 2^-k, every partial sum is exact, and the token follows from the Philox word."""
+    logits = torch.zeros(3, V, device="cuda")
+    for off in range(8):
+        got = decode_ops.sample_step(logits, seed=11, offset=off).tolist()
+        for row, tok in enumerate(got):
+            word = int(philox.philox4x32(row, off, 0, 3, 11, 0)[0])
+            u = np.float32(np.float32((word >> 8) + 0.5) * np.float32(2.0 ** -24))
+            assert tok == math.ceil(float(u) * V) - 1
+
+
+@pytest.mark.parametrize("V", [1, 3, 4, 511, 2048, 32003])
+@pytest.mark.parametrize("shift", [0, 1, 2])
+def test_greedy_token_is_the_first_of_the_largest(V, shift):
+    g = torch.Generator(device="cuda").manual_seed(V)
+    flat = torch.randint(-9, 10, (4 * (V + 5) + shift,), device="cuda", generator=g).float()
+    logits = flat[shift:].view(4, V + 5)[:, :V]
+    got = decode_ops.sample_step(logits, do_sample=False).tolist()
+    assert got == [r.index(max(r)) for r in logits.tolist()]
+
+
 @pytest.mark.parametrize("V", [7, 512, 2049, 32000, 51200])
 @pytest.mark.parametrize("top_k,top_p", [(None, None), (40, None), (None, 0.9), (300, 0.6)])
 def test_sampler_forms_agree(V, top_k, top_p):
@@ -146,7 +169,7 @@ def test_sample_step_marks_finished_rows():
 
 @pytest.mark.parametrize("sample", [False, True])
 def test_generate_stops_rows_at_an_end_of_sequence_id(sample):
-    """The step that is queued before the host sees a token changes nothing: rows end with their first EOS id."""
+    """Rows end with their first EOS id."""
     m = _models()["opt"]().init_random_fast(3, std=0.05)
     g = torch.Generator().manual_seed(4)
     ids = torch.randint(4, 500, (3, 20), generator=g)
