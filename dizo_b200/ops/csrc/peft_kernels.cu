@@ -11,6 +11,39 @@ namespace dz {
 
 constexpr int LORA_MAX_R = 16;
 
+// Small matrices: one row of W per thread, so that every load of the launch is independent of the others.  Us, this kernel /
+// the one below: 768 x 768, rank 2 1.8 / 2.1, rank 8 2.3 / 2.7; 1536 x 1536, rank 8 4.2 / 4.7; 2048 x 2048, rank 1 3.1 / 3.5,
+// rank 4 3.9 / 4.3, rank 8 5.5 / 5.3; 2560 x 2560, rank 1 4.3 / 4.3, rank 4 5.9 / 5.3.
+template <int R>
+__global__ void __launch_bounds__(256)
+lora_merge_row_kernel(const __nv_bfloat16* __restrict__ W, long long ldw,
+                  const __nv_bfloat16* __restrict__ A, long long lda,   // [R, K]
+                  const __nv_bfloat16* __restrict__ B, long long ldb,   // [N, R]
+                  __nv_bfloat16* __restrict__ out, long long ldo, int N, int K, float s) {
+  // grid: (ceil(K / 2048), N); each thread owns 8 consecutive k of one row n
+  const int n = blockIdx.y;
+  const int k0 = (blockIdx.x * 256 + threadIdx.x) * 8;
+  if (k0 >= K) return;
+  float b[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) b[r] = s * __bfloat162float(B[(long long)n * ldb + r]);
+  uint4 w = *reinterpret_cast<const uint4*>(W + (long long)n * ldw + k0);
+  float v[8] = {bf16_lo(w.x), bf16_hi(w.x), bf16_lo(w.y), bf16_hi(w.y),
+                bf16_lo(w.z), bf16_hi(w.z), bf16_lo(w.w), bf16_hi(w.w)};
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    uint4 a = __ldg(reinterpret_cast<const uint4*>(A + (long long)r * lda + k0));
+    v[0] = fmaf(b[r], bf16_lo(a.x), v[0]); v[1] = fmaf(b[r], bf16_hi(a.x), v[1]);
+    v[2] = fmaf(b[r], bf16_lo(a.y), v[2]); v[3] = fmaf(b[r], bf16_hi(a.y), v[3]);
+    v[4] = fmaf(b[r], bf16_lo(a.z), v[4]); v[5] = fmaf(b[r], bf16_hi(a.z), v[5]);
+    v[6] = fmaf(b[r], bf16_lo(a.w), v[6]); v[7] = fmaf(b[r], bf16_hi(a.w), v[7]);
+  }
+  uint4 o;
+  o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
+  o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
+  if (DZ_STORE_OK(out + (long long)n * ldo + k0, 16)) *reinterpret_cast<uint4*>(out + (long long)n * ldo + k0) = o;
+}
+
 constexpr int LM_THREADS = 128;  // 8 columns each
 constexpr int LM_ROWS = 32;      // most rows of W per CTA
 constexpr int LM_UNROLL = 8;     // rows in flight per thread
@@ -28,29 +61,35 @@ lora_merge_kernel(const __nv_bfloat16* __restrict__ W, long long ldw,
   __shared__ float s_b[LM_ROWS * R];
   const int n0 = blockIdx.y * cta_rows;
   const int rows = min(cta_rows, N - n0);
-  for (int i = threadIdx.x; i < rows * R; i += LM_THREADS)
-    s_b[i] = s * __bfloat162float(B[(long long)(n0 + i / R) * ldb + i % R]);
-  __syncthreads();
   const int k0 = (blockIdx.x * LM_THREADS + threadIdx.x) * 8;
-  if (k0 >= K) return;
-  constexpr bool FLOATS = R <= 8;
-  float af[FLOATS ? R : 1][8];
-  uint4 ap[FLOATS ? 1 : R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(A + (long long)r * lda + k0));
-    if (FLOATS) {
-      af[r][0] = bf16_lo(a.x); af[r][1] = bf16_hi(a.x); af[r][2] = bf16_lo(a.y); af[r][3] = bf16_hi(a.y);
-      af[r][4] = bf16_lo(a.z); af[r][5] = bf16_hi(a.z); af[r][6] = bf16_lo(a.w); af[r][7] = bf16_hi(a.w);
-    } else {
-      ap[r] = a;
-    }
-  }
-  for (int n = 0; n < rows; n += LM_UNROLL) {
-    uint4 w[LM_UNROLL];
+  const bool col_ok = k0 < K;
+  // A and the first rows of W are on their way while s * B is staged: on a small matrix the launch is one such round trip
+  uint4 ap[R], w[LM_UNROLL];
+  auto load_w = [&](int n) {
 #pragma unroll
     for (int u = 0; u < LM_UNROLL; ++u)
       if (n + u < rows) w[u] = *reinterpret_cast<const uint4*>(W + (long long)(n0 + n + u) * ldw + k0);
+  };
+  if (col_ok) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) ap[r] = __ldg(reinterpret_cast<const uint4*>(A + (long long)r * lda + k0));
+    load_w(0);
+  }
+  for (int i = threadIdx.x; i < rows * R; i += LM_THREADS)
+    s_b[i] = s * __bfloat162float(B[(long long)(n0 + i / R) * ldb + i % R]);
+  __syncthreads();
+  if (!col_ok) return;
+  constexpr bool FLOATS = R <= 8;
+  float af[FLOATS ? R : 1][8];
+  if constexpr (FLOATS) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      af[r][0] = bf16_lo(ap[r].x); af[r][1] = bf16_hi(ap[r].x); af[r][2] = bf16_lo(ap[r].y); af[r][3] = bf16_hi(ap[r].y);
+      af[r][4] = bf16_lo(ap[r].z); af[r][5] = bf16_hi(ap[r].z); af[r][6] = bf16_lo(ap[r].w); af[r][7] = bf16_hi(ap[r].w);
+    }
+  }
+  for (int n = 0; n < rows; n += LM_UNROLL) {
+    if (n) load_w(n);
 #pragma unroll
     for (int u = 0; u < LM_UNROLL; ++u) {
       if (n + u >= rows) break;
@@ -92,16 +131,21 @@ extern "C" int dz_lora_merge(const void* W, long long ldw, const void* A, long l
   if ((K & 7) || (ldw & 7) || (lda & 7) || (ldo & 7) || (reinterpret_cast<uintptr_t>(W) & 15) ||
       (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(out) & 15))
     return DZ_ERR_ALIGN;
+  const bool small = (long long)N * K <= (r <= 4 ? 8LL << 19 : 5LL << 19) && N <= 65535;      // 2048^2; between 1536^2 and that
   // 32 rows share a CTA's columns of A while that leaves a few CTAs per SM; smaller matrices are cut finer
   const int cols = (K + LM_THREADS * 8 - 1) / (LM_THREADS * 8);
   int rows = LM_ROWS;
   while (rows > 4 && (long long)cols * ((N + rows - 1) / rows) < 4LL * sm_count()) rows /= 2;
-  if ((N + rows - 1) / rows > 65535) return DZ_ERR_TOO_LARGE;
-  dim3 grid(cols, (N + rows - 1) / rows);
+  if (!small && (N + rows - 1) / rows > 65535) return DZ_ERR_TOO_LARGE;
+  const dim3 grid = small ? dim3((K + 2047) / 2048, N) : dim3(cols, (N + rows - 1) / rows);
   auto w = (const __nv_bfloat16*)W; auto a = (const __nv_bfloat16*)A;
   auto b = (const __nv_bfloat16*)B; auto o = (__nv_bfloat16*)out;
   switch (r) {
-#define DZ_R(RR) case RR: lora_merge_kernel<RR><<<grid, LM_THREADS, 0, stream>>>(w, ldw, a, lda, b, ldb, o, ldo, N, K, scaling, rows); break;
+#define DZ_R(RR)                                                                                                       \
+    case RR:                                                                                                           \
+      if (small) lora_merge_row_kernel<RR><<<grid, 256, 0, stream>>>(w, ldw, a, lda, b, ldb, o, ldo, N, K, scaling);   \
+      else lora_merge_kernel<RR><<<grid, LM_THREADS, 0, stream>>>(w, ldw, a, lda, b, ldb, o, ldo, N, K, scaling, rows); \
+      break;
     DZ_R(1) DZ_R(2) DZ_R(3) DZ_R(4) DZ_R(5) DZ_R(6) DZ_R(7) DZ_R(8)
     DZ_R(9) DZ_R(10) DZ_R(11) DZ_R(12) DZ_R(13) DZ_R(14) DZ_R(15) DZ_R(16)
 #undef DZ_R

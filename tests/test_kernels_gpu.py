@@ -9,6 +9,7 @@ from dizo_b200.ops.attention import attention, attention_reference
 from dizo_b200.ops.llama import rmsnorm
 from dizo_b200.ops.loss import option_ce, token_logprobs, verbalizer_ce
 from dizo_b200.ops.norm import add_rows, embed, gather_rows, layernorm, opt_positions
+from dizo_b200.ops.peft import lora_merge
 from dizo_b200.ops.zo import CHUNK, GammaState, ParamArena, Piece, fill_z, perturb_reference, scalar_diff
 
 pytestmark = pytest.mark.gpu
@@ -69,6 +70,23 @@ def test_attention_large_scores_rescale():
     ref = attention_reference(qkv.float(), H)
     assert (out.float() - ref).abs().max().item() < 0.15
     assert ((out.float() - ref).norm() / ref.norm()).item() < 2e-2
+
+
+# ------------------------------------------------------------------ LoRA merge
+@pytest.mark.parametrize("r", [1, 4, 5, 8, 16])
+@pytest.mark.parametrize("N,K", [(1, 8), (33, 1032), (2048, 2048), (2049, 2048), (1280, 2048), (1281, 2048), (70000, 16)])
+def test_lora_merge(N, K, r):
+    """Both kernels (one row a thread, rows that share the columns of A) on either side of the line between them."""
+    g = torch.Generator(device=DEV).manual_seed(N + K + r)
+    w, a, b = (torch.randn(*s, device=DEV, generator=g).bfloat16() for s in ((N, K), (r, K), (N, r)))
+    y = lora_merge(w, a, b, 0.5)
+    assert torch.equal(y[:7], lora_merge(w[:7], a, b[:7], 0.5))
+    z = w.clone()
+    lora_merge(z, a, b, 0.5, out=z)
+    _sync_ok()
+    assert torch.equal(y, z)
+    ref = w.double() + 0.5 * (b.double() @ a.double())
+    assert ((y.double() - ref).norm() / ref.norm()).item() < 2.0 ** -8      # one rounding to bf16: at most 2^-8 of a value
 
 
 # ------------------------------------------------------------------ norm / embed
