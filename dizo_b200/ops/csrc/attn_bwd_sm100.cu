@@ -333,22 +333,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQKV, const __grid_constant
 constexpr int AP_UNROLL = 4;
 __global__ void __launch_bounds__(256)
 attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                     long long ld, float* __restrict__ dsum, int L, int H, int hd, long long pairs, bool o_wide) {
+                     long long ld, float* __restrict__ dsum, uint32_t L, uint32_t H, int hd, uint32_t pairs, bool o_wide) {
   const int l16 = threadIdx.x & 15;
-  const long long groups = (long long)gridDim.x * (blockDim.x >> 4);
-  const long long g0 = (long long)blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);
+  const uint32_t groups = gridDim.x * (blockDim.x >> 4);
+  const uint32_t g0 = blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);
   const bool col_ok = l16 * 8 < hd;
-  // every lane of a warp makes the same number of turns (the shuffles need all of them)
-  const long long turns = (pairs + groups * AP_UNROLL - 1) / (groups * AP_UNROLL);
-  for (long long t = 0; t < turns; ++t) {
+  // every lane of a warp makes the same number of turns (the shuffles need all of them); pairs < 2^31, so w does not wrap
+  const uint32_t turns = (pairs + groups * AP_UNROLL - 1) / (groups * AP_UNROLL);
+  for (uint32_t t = 0; t < turns; ++t) {
     uint4 a[AP_UNROLL], g[AP_UNROLL];
 #pragma unroll
     for (int u = 0; u < AP_UNROLL; ++u) {
-      const long long w = g0 + (t * AP_UNROLL + u) * groups;
+      const uint32_t w = g0 + (t * AP_UNROLL + u) * groups;
       a[u] = g[u] = make_uint4(0u, 0u, 0u, 0u);
       if (w < pairs && col_ok) {
-        const long long row = w / H;
-        const long long at = row * ld + (w - row * H) * hd + l16 * 8;
+        const uint32_t row = w / H;
+        const long long at = row * ld + (int)(w - row * H) * hd + l16 * 8;
         if (o_wide) {
           a[u] = *reinterpret_cast<const uint4*>(o + at);
         } else {                                     // a context that starts at no 16-byte boundary
@@ -369,11 +369,11 @@ attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* _
       }
 #pragma unroll
       for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-      const long long w = g0 + (t * AP_UNROLL + u) * groups;
+      const uint32_t w = g0 + (t * AP_UNROLL + u) * groups;
       if (l16 == 0 && w < pairs) {
-        const long long row = w / H, hh = w - row * H;
-        const long long bb = row / L, l = row - bb * L;
-        dsum[(bb * H + hh) * L + l] = acc;
+        const uint32_t row = w / H, hh = w - row * H;
+        const uint32_t bb = row / L, l = row - bb * L;
+        dsum[(long long)(bb * H + hh) * L + l] = acc;
       }
     }
   }
@@ -411,10 +411,11 @@ extern "C" int dz_attn_bwd(const void* qkv, long long ld_qkv, int q_col0, int k_
   const long long rows = (long long)B * L;
   {
     const long long pairs = rows * H;
-    long long blocks = (pairs + 16 * AP_UNROLL - 1) / (16 * AP_UNROLL);
+    if (pairs > 0x7fffffffLL) return DZ_ERR_TOO_LARGE;       // their q | k | v alone, 16 columns a head, would be 206 GB
+    long long blocks = (pairs + 15) / 16;                    // one pair per half-warp until the chip is full
     if (blocks > 8LL * sm_count()) blocks = 8LL * sm_count();
     attn_bwd_prep_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, ld_out,
-                                                              dsum, L, H, hd, pairs,
+                                                              dsum, L, H, hd, (uint32_t)pairs,
                                                               !(reinterpret_cast<uintptr_t>(out) & 15));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_rc(e);
