@@ -26,8 +26,8 @@
 
 namespace dz {
 
-constexpr int DA_THREADS = 256;
-constexpr int DA_WARPS = DA_THREADS / 32;
+constexpr int DA_WARPS = 8;
+constexpr int DA_FEW_KEYS = 64;
 constexpr int DA_UNROLL = 4;      // keys in flight per lane group
 
 __device__ __forceinline__ void unpack8(const uint4& r, float (&f)[8]) {
@@ -35,15 +35,15 @@ __device__ __forceinline__ void unpack8(const uint4& r, float (&f)[8]) {
   f[4] = bf16_lo(r.z); f[5] = bf16_hi(r.z); f[6] = bf16_lo(r.w); f[7] = bf16_hi(r.w);
 }
 
-// LPK: lanes per key (8 columns each).  grid (H * splits, B), cluster (splits, 1, 1).
-template <int LPK>
-__global__ void __launch_bounds__(DA_THREADS)
+// LPK: lanes per key (8 columns each); WARPS of a CTA.  grid (H * splits, B), cluster (splits, 1, 1).
+template <int LPK, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 decode_attn_kernel(const DecodeAttnArgs p) {
   constexpr int KPW = 32 / LPK;               // keys a warp reads at a time
   __shared__ float s_q[128];
   __shared__ float s_kv[2][128];              // the new key and value (append mode)
-  __shared__ float s_m[DA_WARPS], s_l[DA_WARPS];
-  __shared__ float s_acc[DA_WARPS][128];
+  __shared__ float s_m[WARPS], s_l[WARPS];
+  __shared__ float s_acc[WARPS][128];
   __shared__ float s_cta[2 + 128];            // this CTA's (max, sum, weighted V)
   const int rank = (int)blockIdx.x % p.splits, h = (int)blockIdx.x / p.splits, b = blockIdx.y;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -118,9 +118,9 @@ decode_attn_kernel(const DecodeAttnArgs p) {
   const int n = p.n_prefix + cached - first;
   const __nv_bfloat16* kbase = p.kc + seq + (long long)(first - p.n_prefix) * p.ld_row;
   const __nv_bfloat16* vbase = p.vc + seq + (long long)(first - p.n_prefix) * p.ld_row;
-  const int stride = p.splits * DA_WARPS * KPW;
+  const int stride = p.splits * WARPS * KPW;
   // the trip count is the same for every lane of a warp (the shuffles need all of them)
-  for (int jb = (rank * DA_WARPS + warp) * KPW; jb < n; jb += stride * DA_UNROLL) {
+  for (int jb = (rank * WARPS + warp) * KPW; jb < n; jb += stride * DA_UNROLL) {
     uint4 kr[DA_UNROLL], vr[DA_UNROLL];
 #pragma unroll
     for (int u = 0; u < DA_UNROLL; ++u) {
@@ -181,10 +181,10 @@ decode_attn_kernel(const DecodeAttnArgs p) {
   __syncthreads();
   if (tid < hd) {
     float mm = s_m[0];
-    for (int w = 1; w < DA_WARPS; ++w) mm = fmaxf(mm, s_m[w]);
+    for (int w = 1; w < WARPS; ++w) mm = fmaxf(mm, s_m[w]);
     const float ref = mm == -INFINITY ? 0.f : mm;
     float o = 0.f, ll = 0.f;
-    for (int w = 0; w < DA_WARPS; ++w) {
+    for (int w = 0; w < WARPS; ++w) {
       const float f = __expf(s_m[w] - ref);
       o = fmaf(s_acc[w][tid], f, o);
       ll = fmaf(s_l[w], f, ll);
@@ -234,10 +234,15 @@ int decode_attn_launch(DecodeAttnArgs a, int B, int H, bool dependent, cudaStrea
   if (s > by_keys) s = by_keys;
   a.splits = s < 1 ? 1 : s > 8 ? 8 : s;
   const dim3 grid((unsigned)(H * a.splits), (unsigned)B);
-  cudaError_t e = a.hd <= 64
-      ? pdl_launch(decode_attn_kernel<8>, grid, DA_THREADS, 0, stream, a.splits, dependent, a)
-      : pdl_launch(decode_attn_kernel<16>, grid, DA_THREADS, 0, stream, a.splits, dependent, a);
-  return cuda_rc(e);
+  auto launch = [&](auto kern, int threads) {
+    return cuda_rc(pdl_launch(kern, grid, threads, 0, stream, a.splits, dependent, a));
+  };
+  // Few keys and more CTAs than run at once (74 registers: three CTAs of 256 threads an SM): CTAs of four warps, of which
+  // twice as many fit.  Us, 8 / 4 warps: 16 sequences of 32 heads of 128, 16 keys 5.1 / 3.5, 64 keys 5.6 / 4.7; 64 sequences
+  // of 12 heads of 64, one key 4.7 / 3.2.  With more keys it depends: 32 sequences of 40 heads of 128, 301 keys 35.9 / 39.9.
+  const bool few = a.n_prefix + a.kv_len <= DA_FEW_KEYS && (long long)B * H > 2LL * sm_count();
+  if (a.hd <= 64) return few ? launch(decode_attn_kernel<8, 4>, 128) : launch(decode_attn_kernel<8, DA_WARPS>, DA_WARPS * 32);
+  return few ? launch(decode_attn_kernel<16, 4>, 128) : launch(decode_attn_kernel<16, DA_WARPS>, DA_WARPS * 32);
 }
 
 constexpr int SP_THREADS = 512;

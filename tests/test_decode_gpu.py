@@ -10,6 +10,7 @@ from dizo_b200.models.llama import LlamaConfig, LlamaModel
 from dizo_b200.models.opt import OPTConfig, OPTModel, make_batch
 from dizo_b200.ops import _lib, philox
 from dizo_b200.ops import decode as decode_ops
+from dizo_b200.ops.attention import decode_attention_reference
 
 pytestmark = pytest.mark.gpu
 
@@ -115,6 +116,22 @@ def test_decode_attention_over_rows_off_a_16_byte_boundary(shift):
     ref = decode_ops.decode_attention(q, k.clone(), v.clone(), n - 1, H, None, pk.clone(), pv.clone())
     _lib.check_device_errors()
     assert torch.equal(y, ref)
+
+
+@pytest.mark.parametrize("B,H,hd", [(16, 19, 64), (31, 10, 80), (64, 5, 128)])
+@pytest.mark.parametrize("n", [1, 7, 59, 60, 400])
+def test_decode_attention_of_many_heads(B, H, hd, n):
+    """More (sequence, head) pairs than run at once, around the number of keys (64, prefix rows among them) up to which a CTA
+    has four warps."""
+    g = torch.Generator(device="cuda").manual_seed(n + hd)
+    q, k, v = (torch.randn(*s, device="cuda", generator=g).bfloat16() for s in ((B, H * hd), (B, n, H * hd), (B, n, H * hd)))
+    pk, pv = (torch.randn(5, H * hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    pad = torch.randint(0, n, (B,), device="cuda", dtype=torch.int32, generator=g)
+    y = decode_ops.decode_attention(q, k, v, n, H, pad, pk, pv)
+    _lib.check_device_errors()
+    ref = decode_attention_reference(q.float(), k.float(), v.float(), n, H, pad, pk.float(), pv.float())
+    # one rounding to bf16 (at most 2^-8 of a value) beside fp32 sums and exponentials
+    assert ((y.float() - ref).norm() / ref.norm()).item() < 2.0 ** -8
 
 
 @pytest.mark.parametrize("V", [1024, 4096, 32768, 65536])
