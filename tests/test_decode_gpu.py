@@ -10,14 +10,15 @@ from dizo_b200.models.llama import LlamaConfig, LlamaModel
 from dizo_b200.models.opt import OPTConfig, OPTModel, make_batch
 from dizo_b200.ops import _lib, philox
 from dizo_b200.ops import decode as decode_ops
+from dizo_b200.ops import llama as llama_ops
 from dizo_b200.ops.attention import decode_attention_reference
 
 pytestmark = pytest.mark.gpu
 
 
-def _models():
-    opt = dict(vocab_size=520, hidden_size=160, num_hidden_layers=3, ffn_dim=328, max_position_embeddings=256)
-    lla = dict(vocab_size=520, hidden_size=512, num_hidden_layers=2, intermediate_size=712, max_position_embeddings=256)
+def _models(**kw):
+    opt = dict(vocab_size=520, hidden_size=160, num_hidden_layers=3, ffn_dim=328, max_position_embeddings=256) | kw
+    lla = dict(vocab_size=520, hidden_size=512, num_hidden_layers=2, intermediate_size=712, max_position_embeddings=256) | kw
     return {
         "opt": lambda: OPTModel(OPTConfig(num_attention_heads=2, **opt), "cuda", torch.bfloat16),
         "opt-post": lambda: OPTModel(OPTConfig(num_attention_heads=10, do_layer_norm_before=False, word_embed_proj_dim=64,
@@ -54,8 +55,8 @@ def test_native_step_equals_block_by_block(name, B, L):
         tok = torch.full((B,), 7 + t, dtype=torch.int32, device="cuda")
         a, b = (d.step(tok, pos + t, batch.pad_left) for d in decs)
         _lib.check_device_errors()
-        # the same kernels on the same operands: K / V append and attention sum the same keys, with the newest key taken
-        # from registers instead of the cache (another order of fp32 sums); LLaMA's SwiGLU is the same launch
+        # the same operands in another order of fp32 sums: the newest key comes from registers instead of the cache, a step of
+        # up to four sequences takes its products (LLaMA's SwiGLU among them) through gemv.cu, others split K differently
         assert ((a - b).norm() / b.norm()).item() < 2 * 2.0 ** -8
         for x, y in zip(decs[0].k + decs[0].v, decs[1].k + decs[1].v):
             x, y = x[:, :L + t + 1].float(), y[:, :L + t + 1].float()
@@ -65,6 +66,40 @@ def test_native_step_equals_block_by_block(name, B, L):
         d.reorder(index)
     a, b = (d.step(tok, pos + 3, batch.pad_left[index]) for d in decs)
     assert ((a - b).norm() / b.norm()).item() < 2 * 2.0 ** -8
+
+
+@pytest.mark.parametrize("name", ["opt", "opt-adapters", "llama", "llama-prefix"])
+@pytest.mark.parametrize("B,L", [(1, 600), (2, 330), (3, 330), (4, 700), (7, 301), (64, 70)])
+def test_step_attends_to_all_keys(name, B, L):
+    """The attention inside a step (cache append, keys shared by up to 8 CTAs, products for 1 to 4 rows in registers) against
+    the fp32 statement over the cache it leaves, with padding longer than one CTA's share."""
+    m = _models(num_hidden_layers=1, max_position_embeddings=1024)[name]().init_random_fast(3, std=0.2)
+    cfg, P = m.config, m.num_prefix
+    d, H = cfg.hidden_size, cfg.num_attention_heads
+    mask = torch.ones(B, L, dtype=torch.long)
+    for i in range(B):
+        mask[i, :i * L // (B + 1)] = 0
+    batch = make_batch(torch.randint(4, 500, (B, L), generator=torch.Generator().manual_seed(B * L)), mask).to("cuda")
+    dec = _Decoder(m, B, L + 3)
+    dec.prefill(batch)
+    pos = (mask.sum(1).cuda() + 2).to(torch.int32)
+    for t in range(L, L + 2):
+        dec.step(torch.arange(B, device="cuda", dtype=torch.int32) + t, pos + t - L, batch.pad_left)
+        _lib.check_device_errors()
+        _, _, qkv, ctx, _ = (w.float().cpu() for w in dec.plan._ws)
+        if isinstance(m, LlamaModel):
+            qkv = llama_ops.rope_qkv_reference(qkv, 1, P + t, H, cfg.num_key_value_heads, d // H, cfg.rope_theta)
+            qkv = qkv.bfloat16().float()
+        k, v = dec.k[0].float().cpu(), dec.v[0].float().cpu()
+        # a rotated value may fall on the other side of a rounding to bf16 (2^-7 of it at most); v and unrotated k are copies
+        tol = 2.0 ** -7 if isinstance(m, LlamaModel) else 0.0
+        assert ((k[:, t] - qkv[:, d:2 * d]).abs() <= tol * k[:, t].abs() + tol * 1e-3).all()
+        assert torch.equal(v[:, t], qkv[:, 2 * d:])
+        w = m._layer_weights(0, m._resolver(0, None, None, 0))
+        pk, pv = (None, None) if w.prefix_k is None else (w.prefix_k.float().cpu(), w.prefix_v.float().cpu())
+        ref = decode_attention_reference(qkv[:, :d], k, v, t + 1, H, batch.pad_left.cpu(), pk, pv)
+        # one rounding to bf16 (at most 2^-8 of a value) and, where q is rotated, its own
+        assert ((ctx - ref).norm() / ref.norm()).item() < 2.0 ** -7
 
 
 @pytest.mark.parametrize("name", ["opt", "llama"])
