@@ -31,11 +31,12 @@ int dz_attn_fwd(const void* qkv, long long ld_qkv, int q_col0, int k_col0, int v
 
 using namespace dz;
 
-// Whether the swapped-operand, K-split kernel (skinny_sm100.cu) takes a product.  Up to 16 rows it always wins (one row,
-// us, 128-row tiles / skinny: N 2048 K 8192 32.9 / 10.3, N 50272 K 2048 57.6 / 36.1).  With more rows its wider activation
-// operand costs L2 traffic per tile of W, which only K splitting makes up for: at 32 rows N 32000 K 4096 50.2 / 48.1 but
-// N 50272 K 2048 40.6 / 42.8; at 64 rows N 2048 K 8192 31.9 / 13.7, N 8192 K 2048 12.4 / 11.9, but N 16384 K 4096 29.2 /
-// 29.6 and N 50272 K 2048 40.4 / 49.5.
+// Whether the swapped-operand, K-split kernel (skinny_sm100.cu) takes a product.  Up to 16 rows it, or gemv.cu ahead of it, won
+// on each of the 36 weight shapes measured (N 768 to 50272, K 768 to 20480): 1.22 to 4.0 times as fast as 128-row tiles with
+// 1 to 8 rows, 1.10 to 3.3 with 16 (one row, us: N 2048 K 8192 32.9 / 10.3, N 50272 K 2048 57.6 / 36.1).  With more rows its
+// wider activation operand costs L2 traffic per tile of W, which only K splitting makes up for: at 32 rows N 32000 K 4096
+// 50.2 / 48.1 but N 50272 K 2048 40.6 / 42.8; at 64 rows N 2048 K 8192 31.9 / 13.7, N 8192 K 2048 12.4 / 11.9, but N 16384
+// K 4096 29.2 / 29.6 and N 50272 K 2048 40.4 / 49.5.
 static bool skinny_pays(int M, int N) {
   const int tiles = (N + 127) / 128;
   return M <= 16 || (M <= 32 && tiles <= 296) || (M <= 64 && tiles <= 74);

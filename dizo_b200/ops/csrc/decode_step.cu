@@ -169,7 +169,7 @@ extern "C" int dz_decode_step(const void* plan, const void* const* k_cache, cons
     const bool dep = !first;
     first = false;
     if (p.vector) return gemv_launch(W, K, X, K, a, dep, stream);
-    return skinny_launch(w, x, a, 0, dep, stream);
+    return skinny_launch(w, x, a, 0, true, dep, stream);
   };
   for (int i = 0; i < c.layers; ++i) {
     const LayerPlan& l = p.layers[i];

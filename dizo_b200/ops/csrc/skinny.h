@@ -28,8 +28,9 @@ struct SkinnyArgs {
 // Tensor maps of the operands; the width of the activation box follows from M.
 int skinny_map_w(CUtensorMap* map, const void* W, long long ldw, int rows, int K, bool swiglu);
 int skinny_map_x(CUtensorMap* map, const void* A, long long lda, int M, int K);
-// `splits` 0: chosen from the shape.  `dependent`: programmatic dependent launch.
-int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, int splits, bool dependent,
+// `splits` 0: chosen from the shape and, with `in_step`, so that the next launch of a decoding step fits beside this one.
+// `dependent`: programmatic dependent launch.
+int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, int splits, bool in_step, bool dependent,
                   cudaStream_t stream);
 
 // One to four rows without tensor cores (gemv.cu), where gemv_takes(); worth it where gemv_pays().

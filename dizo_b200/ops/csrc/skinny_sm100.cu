@@ -269,7 +269,7 @@ static int launch_nb(const CUtensorMap& tmW, const CUtensorMap& tmX, const Skinn
   return cuda_rc(e);
 }
 
-int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, int splits, bool dependent,
+int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, int splits, bool in_step, bool dependent,
                   cudaStream_t stream) {
   const int cols = a.act == 3 ? SK_BM / 2 : SK_BM;
   const int nb = sk_nb(a.M);
@@ -278,7 +278,7 @@ int skinny_launch(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyArgs a, 
   if (tiles_ll * 8 > 0x7fffffffLL) return DZ_ERR_TOO_LARGE;
   const int tiles = (int)tiles_ll;
   a.num_kb = (a.K + SK_BK - 1) / SK_BK;
-  if (splits <= 0) splits = choose_splits(tiles, a.num_kb, a.w_static != 0);
+  if (splits <= 0) splits = choose_splits(tiles, a.num_kb, in_step);
   if (splits > 8) splits = 8;
   a.kb_per_cta = (a.num_kb + splits - 1) / splits;
   a.splits = (a.num_kb + a.kb_per_cta - 1) / a.kb_per_cta;     // no CTA without a K block
@@ -319,5 +319,5 @@ extern "C" int dz_gemm_skinny(const void* A, long long lda, const void* W, long 
   if (rc) return rc;
   rc = skinny_map_x(&tmX, A, lda, M, K);
   if (rc) return rc;
-  return skinny_launch(tmW, tmX, a, splits, true, stream);
+  return skinny_launch(tmW, tmX, a, splits, false, true, stream);
 }
