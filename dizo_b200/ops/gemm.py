@@ -132,7 +132,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, a
            tile_n: int = 0) -> torch.Tensor:
     """x [..., K] (bf16), w [N, K] (bf16) -> [..., N] in ``out_dtype`` (bf16 or fp32).
 
-    ``tile_n``: 0 = choose (``dz_linear`` in ``csrc/block_forward.cu``), 128 / 256 = one-SM kernel with that tile width, 512 = two-SM kernel."""
+    ``tile_n``: 0 = choose (``dz_linear`` in ``csrc/block_forward.cu``), 128 / 256 = one-SM kernel with that tile width,
+    512 = two-SM kernel."""
     if not x.is_cuda:
         y = linear_reference(x, w, bias, act, residual, scale, out_dtype)
         if out is not None:
